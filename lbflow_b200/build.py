@@ -26,7 +26,8 @@ NVCC = os.environ.get('NVCC', '/usr/local/cuda/bin/nvcc')
 ARCH = ['-gencode', 'arch=compute_100a,code=sm_100a']
 NVFLAGS = ['-std=c++17', '-O3', '-lineinfo', '--expt-relaxed-constexpr', '-Xcompiler', '-fPIC',
            '-Xcompiler', '-O3'] + ARCH
-CUDA_UNITS = ['engine.cu', 'scsp_launch.cu', 'color_launch.cu', 'noalloc.cu', 'batch.cu', 'conv.cu', 'darcy.cu']
+CUDA_UNITS = ['color_fp16.cu', 'color_bf16.cu', 'color_fp64.cu', 'color_fp32.cu', 'color_launch.cu', 'engine.cu',
+              'scsp_launch.cu', 'noalloc.cu', 'batch.cu', 'conv.cu', 'darcy.cu']
 HOST_UNITS = ['main.cpp', 'prm.cpp', 'io.cpp', 'simulation.cpp']
 LIBNAME = 'liblbflow_b200.so'
 

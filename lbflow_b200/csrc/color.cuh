@@ -135,12 +135,11 @@ __device__ __forceinline__ void color_pull(const Grid& g, const typename S::T* _
         if constexpr (IsPacked<S>::value) S::load_pair(fin, off, nblk, q, rho_bar, a, b);
         else { a = S::load(fin + off, q, R(0)); b = S::load(fin1 + off, q, R(0)); }
     };
-    {
-        R a, b;
-        load2(i, 0, a, b);
-        sink(0, a, b, i);
-    }
     if constexpr (!PULL) {
+        pdl_wait();
+        R a0, b0;
+        load2(i, 0, a0, b0);
+        sink(0, a0, b0, i);
 #pragma unroll
         for (int q = 1; q < L::Q; ++q) {
             R a, b;
@@ -150,6 +149,10 @@ __device__ __forceinline__ void color_pull(const Grid& g, const typename S::T* _
     } else {
         uint32_t src[L::Q];
         const uint32_t mask = pull_sources<L, (sizeof(R) == 4)>(g, x, y, z, src);
+        pdl_wait();
+        R a0, b0;
+        load2(i, 0, a0, b0);
+        sink(0, a0, b0, i);
 #pragma unroll
         for (int q = 1; q < L::Q; ++q) {
             const bool fluid = (mask >> q) & 1u;
@@ -225,6 +228,7 @@ color_phase(const Grid g, const Film film, const typename S::T* __restrict__ fin
             double* __restrict__ phid, uint32_t* __restrict__ err, const double rho_bar)
 {
     using R = typename S::R;
+    pdl_trigger();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= g.nf) return;
     int x, y, z;
@@ -575,10 +579,12 @@ color_collide(const Grid g, const Film film, const Force F, const ColorParams P,
     // populations in ascending order, so the highest nodes' lines are the
     // ones still in L2, and the next step's pass 1 starts with the lowest
     // nodes, the last ones written here.
+    pdl_trigger();
     const uint32_t i = (gridDim.x - 1 - blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= g.nf) return;
     int x, y, z;
     unpack(__ldg(&g.coord[i]), x, y, z);
+    pdl_wait();
     R gr[3], norm;
     color_gradient_dense<L, R>(g, W, phid, i, x, y, z, gr, norm);
     if constexpr (FILM) {
@@ -697,6 +703,7 @@ color_zou_he_phase(const Grid g, const Film film, const ZouHe z, const typename 
                    double* __restrict__ phid, uint32_t* __restrict__ err, const double rho_bar)
 {
     using R = typename S::R;
+    pdl_trigger();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= z.n) return;
     uint32_t i;
@@ -729,6 +736,7 @@ color_zou_he_collide(const Grid g, const Film film, const Force F, const ColorPa
                      const double* __restrict__ phid, Macros mo, const int out, uint32_t* __restrict__ err)
 {
     using R = typename S::R;
+    pdl_trigger();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= z.n) return;
     uint32_t i;

@@ -60,6 +60,24 @@ cudaError_t device_pool(int device, cudaMemPool_t* pool);
 // Message returned by lbf_last_error(NULL) (calls without an engine).
 void set_global_error(const std::string& msg);
 
+// Launch with programmatic stream serialization: the kernel may start before
+// the previous kernel of the stream has completed and calls pdl_wait() before
+// it touches anything an earlier kernel writes or reads.
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t s, A&&... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline unsigned blocks_for(uint32_t n, unsigned threads) { return (n + threads - 1) / threads; }
 
 }  // namespace lbf

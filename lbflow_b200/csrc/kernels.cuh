@@ -57,6 +57,17 @@ struct Macros {                 // compact per-node outputs, stride nfp
     double* indadj;             // color: indicator of the step before a report
 };
 
+// Programmatic dependent launch (every step kernel is launched with it): a
+// block first lets the next step's kernel be scheduled, looks its pull sources
+// up in data that never changes after creation, and only then waits for the
+// previous kernels of the stream to complete and be visible.  The launch gap,
+// the occupancy lookups and the previous step's last, partly filled round of
+// blocks then overlap.  Both are no-ops in a kernel launched without it.
+// Microseconds per step without -> with: FP64 48^3 (24 k nodes) 6.2 -> 4.8,
+// 96^3 12.4 -> 9.5, 256^3 (3.7 M) 186.8 -> 184.1; FP16 192^3 51.1 -> 48.3.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ int wrap(int v, int n) { return v < 0 ? v + n : (v >= n ? v - n : v); }
 
 __device__ __forceinline__ void unpack(uint32_t c, int& x, int& y, int& z)
@@ -311,15 +322,18 @@ __device__ __forceinline__ void gather(const Grid& g, const typename S::T* __res
     // Element offsets stay 32-bit (phases * Q * nfp < 2^32 is checked at
     // creation); only the final address is 64-bit.
     const uint32_t nfp = g.nfp;
-    f[0] = load_pop<S>(fin + i, 0, rho0, ein, i);
     nbr[0] = i;
     if (!PULL) {
+        pdl_wait();
+        f[0] = load_pop<S>(fin + i, 0, rho0, ein, i);
 #pragma unroll
         for (int q = 1; q < L::Q; ++q) { f[q] = load_pop<S>(fin + (q * nfp + i), q, rho0, ein, i); nbr[q] = 0; }
         return;
     }
     uint32_t src[L::Q];
     const uint32_t mask = pull_sources<L, UNIFORM>(g, x, y, z, src);
+    pdl_wait();
+    f[0] = load_pop<S>(fin + i, 0, rho0, ein, i);
 #pragma unroll
     for (int q = 1; q < L::Q; ++q) {
         const bool fluid = (mask >> q) & 1u;
@@ -589,6 +603,7 @@ scsp_step(const Grid g, const Force F, const ScspParams P,
     // The node order alternates between steps: a step that runs in the
     // opposite order to the previous one starts with the nodes whose
     // populations that step wrote last, which are still in L2.
+    pdl_trigger();
     const uint32_t blk = P.reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const uint32_t i = blk * blockDim.x + threadIdx.x;
     if (i >= g.nf) return;
@@ -694,6 +709,7 @@ scsp_zou_he(const Grid g, const ScspParams P, const ZouHe z,
             const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
 {
     using R = typename S::R;
+    pdl_trigger();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= z.n) return;
     const uint32_t i = __ldg(&z.node[k]);

@@ -15,7 +15,8 @@ void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
     if (blocks == 0) return;
     (void)mrt;   // the collision rates (SRT or MRT) are in a.P.rate
     if (pull)
-        scsp_step<L, S, true><<<blocks, threads, 0, a.stream>>>(a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout);
+        launch_pdl(scsp_step<L, S, true>, blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein,
+                   a.eout);
     else
         scsp_step<L, S, false><<<blocks, threads, 0, a.stream>>>(a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout);
 }
@@ -38,9 +39,8 @@ void zou_he(const ScspLaunch& a, const ZouHe& z)
     using T = typename S::T;
     const unsigned threads = 128, blocks = blocks_for(z.n, threads);
     if (blocks == 0) return;
-    scsp_zou_he<L, S><<<blocks, threads, 0, a.stream>>>(a.g, a.P, z, static_cast<const T*>(a.fin),
-                                                         static_cast<T*>(a.fout), a.mo, a.out, a.err,
-                                                         a.ein, a.eout);
+    launch_pdl(scsp_zou_he<L, S>, blocks, threads, a.stream, a.g, a.P, z, static_cast<const T*>(a.fin),
+               static_cast<T*>(a.fout), a.mo, a.out, a.err, a.ein, a.eout);
 }
 
 template <class L>
