@@ -64,8 +64,10 @@ enum {
     LBF_ERR_COMPONENT = 1u << 1,  /* negative component density (color) */
     LBF_ERR_TAU = 1u << 2,        /* local relaxation time <= 0.5 (color) */
     LBF_ERR_VELOCITY = 1u << 3,   /* non-finite velocity (color) */
-    LBF_ERR_OUTPUT = 1u << 4      /* non-finite population met by
+    LBF_ERR_OUTPUT = 1u << 4,     /* non-finite population met by
                                      lbf_populations_dense_async */
+    LBF_ERR_WAIT = 1u << 5        /* a multi-step launch gave up waiting for a
+                                     neighbouring node */
 };
 
 /* lbf_step flags: what the LAST step of the call also writes. */

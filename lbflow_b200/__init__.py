@@ -30,7 +30,8 @@ ERR_BITS = {1: 'Non-finite or non-positive fluid density.',
             2: 'Negative component density outside roundoff tolerance.',
             4: 'Invalid local relaxation time.',
             8: 'Non-finite fluid velocity.',
-            16: 'Non-finite post-collision population; no restart will be written.'}
+            16: 'Non-finite post-collision population; no restart will be written.',
+            32: 'A multi-step launch gave up waiting for a neighbouring node.'}
 
 
 class LbfError(RuntimeError):

@@ -62,6 +62,10 @@ struct lbf_engine {
     bool initialized = false;
     uint32_t steps = 0;             // pull steps launched (seeds the 16-bit stochastic rounding)
     uint32_t pulls = 0;             // pull steps launched (alternates the step kernel's node order)
+    void* words = nullptr;          // tagged words of the resident steps (allocated on first use)
+    uint32_t tag = 0;               // step number of the last resident step
+    bool resident_asked = false;    // resident_nodes is known
+    uint32_t resident_nodes = 0;    // largest geometry the resident steps take
     uint64_t bytes = 0;
     std::string last_error;
 };
@@ -1106,7 +1110,7 @@ void lbf_destroy(lbf_engine* e)
                     e->rho0, e->rho1, e->u, e->uprev, e->uadj, e->ind, e->indprev, e->indadj,
                     e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red,
                     e->zh_node, e->zh_code, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
-                    e->stage, e->phid, e->solid_f[0], e->solid_f[1]};
+                    e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, e->stream);
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->h_red) cudaFreeHost(e->h_red);
@@ -1268,6 +1272,64 @@ int lbf_add_density(lbf_engine* e, const float* drho)
     return LBF_OK;
 }
 
+namespace {
+// Whether this engine's steps run in one resident launch (resident.cuh): a
+// single-phase engine without boundary planes, block exponents or solid
+// populations, all of whose nodes the device holds at once.
+bool resident_ok(lbf_engine* e)
+{
+    if (e->cfg.model != LBF_MODEL_SCSP || e->cfg.storage == LBF_STORE_BFP16 || e->zh.n || e->solid_f[0] || !e->nf)
+        return false;
+    if (!e->resident_asked) {
+        e->resident_asked = true;
+        if (scsp_resident_nodes(e->D, (int)e->cfg.storage, &e->resident_nodes) != cudaSuccess) {
+            cudaGetLastError();
+            e->resident_nodes = 0;
+        }
+    }
+    if (e->nf > e->resident_nodes) return false;
+    // A replayed launch would repeat its step numbers: while the caller
+    // captures the stream, one launch per step.
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(e->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
+// Queues the steps; false, with nothing queued, where the device cannot take
+// the launch or the words' memory: the caller then launches step by step.
+bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
+{
+    const size_t bytes = 2 * (size_t)(e->Q - 1) * e->nfp * (e->cfg.storage == LBF_STORE_FP64 ? 16 : 8);
+    bool clear = nsteps >= 0xffffffffu - e->tag;   // step numbers start over: no word may still hold one
+    if (!e->words) {
+        unsigned long long* w = nullptr;
+        if (dalloc(e, &w, bytes / 8)) {
+            cudaGetLastError();
+            e->resident_nodes = 0;
+            return false;
+        }
+        e->words = w;
+        clear = true;
+    }
+    if (clear) {
+        if (cudaMemsetAsync(e->words, 0, bytes, e->stream) != cudaSuccess) { cudaGetLastError(); return false; }
+        e->tag = 0;
+    }
+    const bool dither = e->cfg.storage == LBF_STORE_FP16 || e->cfg.storage == LBF_STORE_BF16;
+    e->sp.seed = dither ? e->steps + 1 : 0;
+    const ScspLaunch a{grid_of(e), e->force, e->sp, e->f[e->cur], e->f[e->cur ^ 1], macros_of(e), e->err, e->stream,
+                       e->ex[e->cur], e->ex[e->cur ^ 1], out};
+    if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess) {
+        cudaGetLastError();
+        e->resident_nodes = 0;
+        return false;
+    }
+    e->tag += nsteps;
+    if (dither) e->steps += nsteps;
+    e->cur ^= 1;
+    return true;
+}
+}  // namespace
+
 int lbf_step(lbf_engine* e, uint32_t nsteps, uint32_t flags)
 {
     if (!e) return fail(e, LBF_EINVAL, "NULL engine");
@@ -1275,6 +1337,7 @@ int lbf_step(lbf_engine* e, uint32_t nsteps, uint32_t flags)
     int rc = setdev(e);
     if (rc) return rc;
     const int out = (flags & LBF_STEP_MACROS ? kOutMacros : 0) | (flags & LBF_STEP_ADJACENT ? kOutAdjacent : 0);
+    if (nsteps > 1 && resident_ok(e) && resident_steps(e, nsteps, out)) return LBF_OK;
     for (uint32_t s = 0; s < nsteps; ++s) launch_step(e, true, s + 1 == nsteps ? out : 0);
     LBF_CK(e, cudaGetLastError());
     return LBF_OK;

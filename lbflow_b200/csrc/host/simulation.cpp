@@ -73,6 +73,7 @@ void Simulation::checkDevice() const
     if (bits & LBF_ERR_COMPONENT) throw std::runtime_error("Negative component density outside roundoff tolerance.");
     if (bits & LBF_ERR_TAU) throw std::runtime_error("Invalid local relaxation time.");
     if (bits & LBF_ERR_VELOCITY) throw std::runtime_error("Non-finite fluid velocity.");
+    if (bits & LBF_ERR_WAIT) throw std::runtime_error("A multi-step launch gave up waiting for a neighbouring node.");
 }
 
 Simulation::Simulation(const Params& p) : p_(p)

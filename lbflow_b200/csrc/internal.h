@@ -5,6 +5,7 @@
 #include <string>
 #include "kernels.cuh"
 #include "color.cuh"
+#include "resident.cuh"
 
 namespace lbf {
 
@@ -44,6 +45,10 @@ void launch_scsp_init(int dims, int storage, const Grid& g, const Force& F, doub
                       void* f, int8_t* eout, cudaStream_t s);
 // Zou-He PB/VB boundary pass of one pull step (after launch_scsp, same buffers).
 void launch_scsp_zou_he(int dims, int storage, const ScspLaunch& a, const ZouHe& z);
+// All steps of a call in one launch (resident.cuh): a.out applies to the last.
+// The caller keeps nf within scsp_resident_nodes (0 where unsupported).
+cudaError_t launch_scsp_resident(int dims, int storage, const ScspLaunch& a, const Resident& r);
+cudaError_t scsp_resident_nodes(int dims, int storage, uint32_t* nodes);
 void launch_scsp_add_density(int dims, int storage, const Grid& g, const float* drho, void* f, int8_t* eio,
                              double rho0, cudaStream_t s);
 void launch_scsp_init_eq(int dims, int storage, const Grid& g, const Force& F, double rho0, const float* fields,

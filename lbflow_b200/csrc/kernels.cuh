@@ -26,6 +26,7 @@ enum : uint32_t {
     kErrTau       = 1u << 2,  // local relaxation time <= 0.5 (colorfluid.cpp:269-270)
     kErrVelocity  = 1u << 3,  // non-finite velocity (colorfluid.cpp:282-283)
     kErrOutput    = 1u << 4,  // non-finite population in a dense checkpoint copy (simulator.cpp:327-333)
+    kErrWait      = 1u << 5,  // a multi-step launch gave up waiting for a neighbour's step
 };
 
 // Output requests for a step kernel.
@@ -129,6 +130,15 @@ __device__ __forceinline__ uint32_t pack_sr(__nv_bfloat16, float hi, float lo, u
     return d;
 }
 
+// Integer hash (lowbias32 of C. Wellons) seeding the per-node rounding stream.
+__device__ __forceinline__ uint32_t hash32(uint32_t x)
+{
+    x ^= x >> 16; x *= 0x7feb352du;
+    x ^= x >> 15; x *= 0x846ca68bu;
+    x ^= x >> 16;
+    return x;
+}
+
 // Shifted 16-bit float storage (H: __half or __nv_bfloat16).
 template <class L, class H> struct StoreShifted16 {
     static constexpr bool blocked = false;
@@ -143,6 +153,11 @@ template <class L, class H> struct StoreShifted16 {
     {
         return __fmul_rn(float(__ldg(p)), ShiftScale<L>::inv(q));
     }
+    // The value that load() gives for these stored bits.
+    __device__ static R from_bits(uint16_t b, int q)
+    {
+        return __fmul_rn(float(*reinterpret_cast<const H*>(&b)), ShiftScale<L>::inv(q));
+    }
     __device__ static void store(T* p, R v, int q, R) { *p = T(v * ShiftScale<L>::scale(q)); }
     // Directions qa (low half) and qb (high half) rounded together; rbits
     // carries 16 random bits for each.
@@ -155,6 +170,27 @@ template <class L, class H> struct StoreShifted16 {
     __device__ static void store_sr1(T* p, R v, int q, uint32_t rbits)
     {
         *reinterpret_cast<uint16_t*>(p) = (uint16_t)pack_sr(H(0.0f), 0.0f, v * ShiftScale<L>::scale(q), rbits);
+    }
+    // The stored bits of all directions of node i (seed != 0): the draws and
+    // pairs of scsp_store.
+    template <class Params>
+    __device__ static void round(const R (&f)[L::Q], uint16_t (&b)[L::Q], const Params& P, uint32_t i)
+    {
+        uint32_t r = hash32((i - P.node0) * 0x9e3779b9u + P.seed);
+#pragma unroll
+        for (int q = 0; q < L::Q; q += 2) {
+            r = r * 1664525u + 1013904223u;
+            const uint32_t ra = r;
+            if (q + 1 < L::Q) {
+                r = r * 1664525u + 1013904223u;
+                const uint32_t d = pack_sr(H(0.0f), f[q + 1] * ShiftScale<L>::scale(q + 1),
+                                           f[q] * ShiftScale<L>::scale(q), __byte_perm(ra, r, 0x7632));
+                b[q] = (uint16_t)d;
+                b[q + 1] = (uint16_t)(d >> 16);
+            } else {
+                b[q] = (uint16_t)pack_sr(H(0.0f), 0.0f, f[q] * ShiftScale<L>::scale(q), ra >> 16);
+            }
+        }
     }
 };
 template <class L> using StoreF16 = StoreShifted16<L, __half>;
@@ -480,32 +516,15 @@ struct ScspParams {
     int reverse = 0;    // blocks in descending node order (alternated every step; see scsp_step)
 };
 
-// Integer hash (lowbias32 of C. Wellons) seeding the per-node rounding stream.
-__device__ __forceinline__ uint32_t hash32(uint32_t x)
-{
-    x ^= x >> 16; x *= 0x7feb352du;
-    x ^= x >> 15; x *= 0x846ca68bu;
-    x ^= x >> 16;
-    return x;
-}
-
-// Update of one fluid node i (the body of scsp_step, shared with the batched
-// kernel).
-template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4)>
-__device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const ScspParams& P,
-                                            const typename S::T* __restrict__ fin,
-                                            typename S::T* __restrict__ fout, const uint32_t i,
-                                            const Macros& mo, const int out, uint32_t* __restrict__ err,
-                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+// Macroscopic variables and collision of node i: f holds the gathered
+// populations and becomes the post-collision ones.
+template <class L, class S>
+__device__ __forceinline__ void scsp_collide(const Grid& g, const Force& F, const ScspParams& P, const uint32_t i,
+                                             typename S::R (&f)[L::Q], const Macros& mo, const int out,
+                                             uint32_t* __restrict__ err)
 {
     using R = typename S::R;
-    int x, y, z;
-    unpack(__ldg(&g.coord[i]), x, y, z);
     const R rho0 = R(P.rho0);
-    R f[L::Q];
-    uint32_t nbr[L::Q];
-    gather<L, S, PULL, UNIFORM>(g, fin, i, x, y, z, f, nbr, rho0, ein);
-
     R Fv[3];
     if (F.uniform) { Fv[0] = R(F.fx); Fv[1] = R(F.fy); Fv[2] = R(F.fz); }
     else {
@@ -550,7 +569,15 @@ __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const
     // and Guo source (simulator.cpp:230-246), relaxed in the two-rate form.
     collide_trt<L, R, false>(f, nullptr, rho - rho0 * R(1.5) * usq, rho0 * R(4.5), rho0 * R(3),
                              u, Fv, uf, R(P.rate.sp), R(P.rate.sm));
+}
 
+// Store of a node's post-collision populations.
+template <class L, class S>
+__device__ __forceinline__ void scsp_store(const Grid& g, const ScspParams& P, typename S::T* __restrict__ fout,
+                                           const uint32_t i, typename S::R (&f)[L::Q], int8_t* __restrict__ eout)
+{
+    using R = typename S::R;
+    const R rho0 = R(P.rho0);
     if constexpr (S::blocked) {
         S::store_blk(fout, g.nfp, i, f, eout);
     } else if constexpr (S::dither) {
@@ -580,6 +607,24 @@ __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const
 #pragma unroll
         for (int q = 0; q < L::Q; ++q) S::store(fout + (q * g.nfp + i), f[q], q, rho0);
     }
+}
+
+// Update of one fluid node i (the body of scsp_step, shared with the batched
+// kernel).
+template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4)>
+__device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const ScspParams& P,
+                                            const typename S::T* __restrict__ fin,
+                                            typename S::T* __restrict__ fout, const uint32_t i,
+                                            const Macros& mo, const int out, uint32_t* __restrict__ err,
+                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+{
+    int x, y, z;
+    unpack(__ldg(&g.coord[i]), x, y, z);
+    typename S::R f[L::Q];
+    uint32_t nbr[L::Q];
+    gather<L, S, PULL, UNIFORM>(g, fin, i, x, y, z, f, nbr, typename S::R(P.rho0), ein);
+    scsp_collide<L, S>(g, F, P, i, f, mo, out, err);
+    scsp_store<L, S>(g, P, fout, i, f, eout);
 }
 
 // Resident 128-thread blocks per SM the step kernel is compiled for.  FP64:

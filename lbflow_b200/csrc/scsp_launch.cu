@@ -55,6 +55,46 @@ void zou_he_storage(int storage, const ScspLaunch& a, const ZouHe& z)
     }
 }
 
+// The resident kernel's launch (nodes = nullptr), or the number of nodes the
+// device holds at once.
+template <class L, class S>
+cudaError_t resident(const ScspLaunch* a, const Resident* r, uint32_t* nodes)
+{
+    using T = typename S::T;
+    constexpr unsigned threads = kResidentThreads;
+    if (nodes) {
+        int dev = 0, sms = 0, per = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, scsp_resident<L, S>, threads, 0);
+        *nodes = (uint32_t)(sms * per) * threads;
+        return e;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks_for(a->g.nf, threads));
+    cfg.blockDim = dim3(threads);
+    cfg.stream = a->stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeCooperative;
+    attr.val.cooperative = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, scsp_resident<L, S>, a->g, a->F, a->P, static_cast<const T*>(a->fin),
+                              static_cast<T*>(a->fout), *r, a->mo, a->out, a->err);
+}
+
+template <class L>
+cudaError_t resident_storage(int storage, const ScspLaunch* a, const Resident* r, uint32_t* nodes)
+{
+    switch (storage) {
+    case LBF_STORE_FP64: return resident<L, StoreF64>(a, r, nodes);
+    case LBF_STORE_FP32: return resident<L, StoreF32<L>>(a, r, nodes);
+    case LBF_STORE_FP16: return resident<L, StoreF16<L>>(a, r, nodes);
+    case LBF_STORE_BF16: return resident<L, StoreBF16<L>>(a, r, nodes);
+    default: return cudaErrorNotSupported;
+    }
+}
+
 template <class L>
 void init_storage(int storage, const Grid& g, const Force& F, double rho0, void* f, int8_t* e, cudaStream_t s)
 {
@@ -116,6 +156,17 @@ void launch_scsp(int dims, int storage, bool mrt, bool pull, int out, const Scsp
 {
     if (dims == 3) dispatch_storage<D3Q19>(storage, mrt, pull, out, a);
     else dispatch_storage<D2Q9>(storage, mrt, pull, out, a);
+}
+
+cudaError_t launch_scsp_resident(int dims, int storage, const ScspLaunch& a, const Resident& r)
+{
+    return dims == 3 ? resident_storage<D3Q19>(storage, &a, &r, nullptr) : resident_storage<D2Q9>(storage, &a, &r, nullptr);
+}
+
+cudaError_t scsp_resident_nodes(int dims, int storage, uint32_t* nodes)
+{
+    return dims == 3 ? resident_storage<D3Q19>(storage, nullptr, nullptr, nodes)
+                     : resident_storage<D2Q9>(storage, nullptr, nullptr, nodes);
 }
 
 void launch_scsp_zou_he(int dims, int storage, const ScspLaunch& a, const ZouHe& z)
