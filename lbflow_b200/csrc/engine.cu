@@ -54,7 +54,7 @@ struct lbf_engine {
     cudaStream_t stream = nullptr;
     Force force{};
     ZouHe zh{};                     // PB/VB boundary nodes (single phase)
-    uint32_t *zh_node = nullptr, *zh_code = nullptr;
+    uint32_t *zh_node = nullptr, *zh_code = nullptr, *zh_bits = nullptr;
     double *zh_value = nullptr, *zh_num = nullptr;
     uint32_t* film_bits[2] = {nullptr, nullptr};   // half-film voxels of phase 0 / 1 (color)
     ScspParams sp{};
@@ -254,11 +254,8 @@ void launch_step(lbf_engine* e, bool pull, int out)
         e->sp.seed = dither && pull ? (++e->steps * 2654435761u) | 1u : 0u;
         e->sp.reverse = pull ? (int)(++e->pulls & 1u) : 0;
         ScspLaunch a{grid_of(e), e->force, e->sp, fin, fout, macros_of(e), e->err, e->stream,
-                     e->ex[e->cur], e->ex[e->cur ^ 1], out};
+                     e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh};
         launch_scsp(e->D, (int)e->cfg.storage, e->cfg.collision == LBF_MRT, pull, out, a);
-        // At t = 0 (no pull) the boundary nodes hold rho0 at rest, which the
-        // main kernel reproduces from their initial populations.
-        if (pull && e->zh.n) launch_scsp_zou_he(e->D, (int)e->cfg.storage, a, e->zh);
     } else {
         // 16-bit storage rounds stochastically with a fresh seed every pull
         // step, as the single-phase path does.
@@ -969,6 +966,15 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
         LBF_CUDA(cudaMemcpyAsync(e->zh_node, zh_node.data(), zh_node.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream));
         LBF_CUDA(cudaMemcpyAsync(e->zh_code, zh_code.data(), zh_code.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream));
         LBF_CUDA(cudaMemcpyAsync(e->zh_value, zh_value.data(), zh_value.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream));
+        std::vector<uint32_t> bits;
+        if (c.model == LBF_MODEL_SCSP) {
+            bits.assign((e->nf + 31) / 32, 0u);
+            for (uint32_t k : zh_node) bits[k >> 5] |= 1u << (k & 31);
+            LBF_ALLOC(e->zh_bits, bits.size());
+            LBF_CUDA(cudaMemcpyAsync(e->zh_bits, bits.data(), bits.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, e->stream));
+            LBF_CUDA(cudaStreamSynchronize(e->stream));
+            e->zh.bits = e->zh_bits;
+        }
         if (c.model == LBF_MODEL_COLOR) {
             LBF_ALLOC(e->zh_num, zh_node.size());
             LBF_CUDA(cudaMemsetAsync(e->zh_num, 0, zh_node.size() * sizeof(double), e->stream));
@@ -1109,7 +1115,7 @@ void lbf_destroy(lbf_engine* e)
     void* ptrs[] = {e->f[0], e->f[1], e->ex[0], e->ex[1], e->occ, e->coord, e->node_label, e->node_phase, e->label_force,
                     e->rho0, e->rho1, e->u, e->uprev, e->uadj, e->ind, e->indprev, e->indadj,
                     e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red,
-                    e->zh_node, e->zh_code, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
+                    e->zh_node, e->zh_code, e->zh_bits, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
                     e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, e->stream);
     if (e->stream) cudaStreamSynchronize(e->stream);
@@ -1317,7 +1323,7 @@ bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
     const bool dither = e->cfg.storage == LBF_STORE_FP16 || e->cfg.storage == LBF_STORE_BF16;
     e->sp.seed = dither ? e->steps + 1 : 0;
     const ScspLaunch a{grid_of(e), e->force, e->sp, e->f[e->cur], e->f[e->cur ^ 1], macros_of(e), e->err, e->stream,
-                       e->ex[e->cur], e->ex[e->cur ^ 1], out};
+                       e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh};
     if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess) {
         cudaGetLastError();
         e->resident_nodes = 0;

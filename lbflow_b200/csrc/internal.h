@@ -20,7 +20,8 @@ struct ScspLaunch {
     cudaStream_t stream;
     const int8_t* ein;   // block exponents of fin (block-scaled storage only)
     int8_t* eout;
-    int out;             // kOutMacros / kOutAdjacent of this step (boundary pass)
+    int out;             // kOutMacros / kOutAdjacent of this step
+    ZouHe zh;            // PB/VB boundary nodes (n = 0: none)
 };
 
 struct ColorLaunch {
@@ -43,8 +44,6 @@ struct ColorLaunch {
 void launch_scsp(int dims, int storage, bool mrt, bool pull, int out, const ScspLaunch& a);
 void launch_scsp_init(int dims, int storage, const Grid& g, const Force& F, double rho0,
                       void* f, int8_t* eout, cudaStream_t s);
-// Zou-He PB/VB boundary pass of one pull step (after launch_scsp, same buffers).
-void launch_scsp_zou_he(int dims, int storage, const ScspLaunch& a, const ZouHe& z);
 // All steps of a call in one launch (resident.cuh): a.out applies to the last.
 // The caller keeps nf within scsp_resident_nodes (0 where unsupported).
 cudaError_t launch_scsp_resident(int dims, int storage, const ScspLaunch& a, const Resident& r);

@@ -635,36 +635,27 @@ __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const
 // fall to 12,800).  FP32 arithmetic (the reduced-precision storages): nine
 // (56 registers, no spill); capped at seven they take 72 registers and run
 // slower (FP32 storage 28,650 -> 26,600, FP16 25,050 -> 24,700).
-template <class S> struct StepBlocks { static constexpr int value = 9; };
-template <> struct StepBlocks<StoreF64> { static constexpr int value = 7; };
-
-template <class L, class S, bool PULL>
-__global__ void __launch_bounds__(128, StepBlocks<S>::value)
-scsp_step(const Grid g, const Force F, const ScspParams P,
-          const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-          Macros mo, const int out, uint32_t* __restrict__ err,
-          const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
-{
-    // The node order alternates between steps: a step that runs in the
-    // opposite order to the previous one starts with the nodes whose
-    // populations that step wrote last, which are still in L2.
-    pdl_trigger();
-    const uint32_t blk = P.reverse ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-    const uint32_t i = blk * blockDim.x + threadIdx.x;
-    if (i >= g.nf) return;
-    scsp_update<L, S, PULL>(g, F, P, fin, fout, i, mo, out, err, ein, eout);
-}
+// With boundary nodes in the same launch FP64 takes five (96 registers, no
+// spill): 161x93x117 with two pressure planes, 537 k nodes, 37.4 us per step;
+// four 39.6, six 40.3, seven 47.4 (the boundary update spills), and a call
+// that is not inlined 70.8.
+template <class S> struct StepBlocks { static constexpr int value = 9, boundary = 9; };
+template <> struct StepBlocks<StoreF64> { static constexpr int value = 7, boundary = 5; };
 
 // ---- Zou-He pressure (PB) and velocity (VB) boundaries ---------------------------
 // SCSP::zouHeBoundary (scsp.cpp:188-275) runs between streaming and the
 // macroscopic update; PB/VB voxels then skip calcMacroVar (scsp.cpp:136-160)
 // and collide with the density and velocity it set, under zero force
-// (forceForIndex is zero for non-GV labels, simulator.cpp:218-228).  The main
-// step kernel treats every fluid node alike; this pass, launched right after
-// it on the same stream, recomputes the boundary nodes from the same input
-// buffer and overwrites their populations and fields.
+// (forceForIndex is zero for non-GV labels, simulator.cpp:218-228).  The step
+// kernel's first blocks update the boundary nodes, one thread per node of a
+// compact list; the other blocks skip those nodes by a bitmap (one word per
+// warp).  A boundary node's update is a long dependent chain on few warps: as
+// a launch of its own after the step it left the rest of the chip idle
+// (161x93x117, 537 k nodes, two pressure planes: FP64 45.4 -> 37.4 us per
+// step, FP32 27.1 -> 16.4).
 struct ZouHe {
     uint32_t n;                          // boundary nodes
+    const uint32_t* __restrict__ bits;   // single phase: bit i of the map is set when node i is one
     const uint32_t* __restrict__ node;   // compact node index
     const uint32_t* __restrict__ code;   // phase << 16 | kind << 8 | dir (dir 1..2D, the lattice direction)
     const double* __restrict__ value;    // PB density or VB speed
@@ -746,17 +737,14 @@ __device__ __forceinline__ typename S::R zou_he_node(typename S::R (&f)[L::Q], u
     return rho;
 }
 
+// Update of the k-th boundary node.
 template <class L, class S>
-__global__ void __launch_bounds__(128)
-scsp_zou_he(const Grid g, const ScspParams P, const ZouHe z,
-            const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-            Macros mo, const int out, uint32_t* __restrict__ err,
-            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+__device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, const ZouHe& z, const uint32_t k,
+                                            const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+                                            const Macros& mo, const int out, uint32_t* __restrict__ err,
+                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
 {
     using R = typename S::R;
-    pdl_trigger();
-    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= z.n) return;
     const uint32_t i = __ldg(&z.node[k]);
     const uint32_t code = __ldg(&z.code[k]);
     const double val = __ldg(&z.value[k]);
@@ -766,6 +754,13 @@ scsp_zou_he(const Grid g, const ScspParams P, const ZouHe z,
     R f[L::Q];
     uint32_t nbr[L::Q];
     gather<L, S, true>(g, fin, i, x, y, zc, f, nbr, rho0, ein);
+
+    // The density check of every node's pulled populations.
+    R pulled = f[0];
+#pragma unroll
+    for (int q = 1; q < L::Q; ++q) pulled += f[q];
+    if (S::shifted) pulled = rho0 + pulled;
+    if (!(pulled > R(0)) || !isfinite(pulled)) atomicOr(err, kErrDensity);
 
     const uint32_t kind = (code >> 8) & 0xffu;
     R u[3];
@@ -838,6 +833,35 @@ scsp_zou_he(const Grid g, const ScspParams P, const ZouHe z,
 #pragma unroll
         for (int q = 0; q < L::Q; ++q) S::store(fout + (q * g.nfp + i), f[q], q, rho0);
     }
+}
+
+// One step of every node.  BOUNDARY: the grid's first `zblocks` blocks update
+// the Zou-He nodes and the others leave them out.
+template <class L, class S, bool PULL, bool BOUNDARY>
+__global__ void __launch_bounds__(128, BOUNDARY ? StepBlocks<S>::boundary : StepBlocks<S>::value)
+scsp_step(const Grid g, const Force F, const ScspParams P,
+          const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+          Macros mo, const int out, uint32_t* __restrict__ err,
+          const int8_t* __restrict__ ein, int8_t* __restrict__ eout, const ZouHe z, const uint32_t zblocks)
+{
+    // The node order alternates between steps: a step that runs in the
+    // opposite order to the previous one starts with the nodes whose
+    // populations that step wrote last, which are still in L2.
+    pdl_trigger();
+    uint32_t b = blockIdx.x, blocks = gridDim.x;
+    if (BOUNDARY) {
+        if (b < zblocks) {
+            const uint32_t k = b * blockDim.x + threadIdx.x;
+            if (k < z.n) scsp_zou_he<L, S>(g, P, z, k, fin, fout, mo, out, err, ein, eout);
+            return;
+        }
+        b -= zblocks;
+        blocks -= zblocks;
+    }
+    const uint32_t i = (P.reverse ? blocks - 1 - b : b) * blockDim.x + threadIdx.x;
+    if (i >= g.nf) return;
+    if (BOUNDARY && ((__ldg(&z.bits[i >> 5]) >> (i & 31)) & 1u)) return;
+    scsp_update<L, S, PULL>(g, F, P, fin, fout, i, mo, out, err, ein, eout);
 }
 
 // t = 0 populations of SCSP::initialize (scsp.cpp:116-134):

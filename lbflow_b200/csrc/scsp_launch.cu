@@ -14,11 +14,18 @@ void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
     const unsigned threads = 128, blocks = blocks_for(a.g.nf, threads);
     if (blocks == 0) return;
     (void)mrt;   // the collision rates (SRT or MRT) are in a.P.rate
-    if (pull)
-        launch_pdl(scsp_step<L, S, true>, blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein,
-                   a.eout);
+    // At t = 0 (no pull) the boundary nodes hold rho0 at rest, which the
+    // ordinary update reproduces from their initial populations.
+    const unsigned zb = pull ? blocks_for(a.zh.n, threads) : 0;
+    if (zb)
+        launch_pdl(scsp_step<L, S, true, true>, zb + blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out,
+                   a.err, a.ein, a.eout, a.zh, zb);
+    else if (pull)
+        launch_pdl(scsp_step<L, S, true, false>, blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err,
+                   a.ein, a.eout, a.zh, 0u);
     else
-        scsp_step<L, S, false><<<blocks, threads, 0, a.stream>>>(a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout);
+        scsp_step<L, S, false, false><<<blocks, threads, 0, a.stream>>>(a.g, a.F, a.P, fin, fout, a.mo, out, a.err,
+                                                                        a.ein, a.eout, a.zh, 0u);
 }
 
 template <class L>
@@ -30,28 +37,6 @@ void dispatch_storage(int storage, bool mrt, bool pull, int out, const ScspLaunc
     case LBF_STORE_BF16: dispatch<L, StoreBF16<L>>(mrt, pull, out, a); break;
     case LBF_STORE_BFP16: dispatch<L, StoreBFP16<L>>(mrt, pull, out, a); break;
     default: dispatch<L, StoreF32<L>>(mrt, pull, out, a); break;
-    }
-}
-
-template <class L, class S>
-void zou_he(const ScspLaunch& a, const ZouHe& z)
-{
-    using T = typename S::T;
-    const unsigned threads = 128, blocks = blocks_for(z.n, threads);
-    if (blocks == 0) return;
-    launch_pdl(scsp_zou_he<L, S>, blocks, threads, a.stream, a.g, a.P, z, static_cast<const T*>(a.fin),
-               static_cast<T*>(a.fout), a.mo, a.out, a.err, a.ein, a.eout);
-}
-
-template <class L>
-void zou_he_storage(int storage, const ScspLaunch& a, const ZouHe& z)
-{
-    switch (storage) {
-    case LBF_STORE_FP64: zou_he<L, StoreF64>(a, z); break;
-    case LBF_STORE_FP16: zou_he<L, StoreF16<L>>(a, z); break;
-    case LBF_STORE_BF16: zou_he<L, StoreBF16<L>>(a, z); break;
-    case LBF_STORE_BFP16: zou_he<L, StoreBFP16<L>>(a, z); break;
-    default: zou_he<L, StoreF32<L>>(a, z); break;
     }
 }
 
@@ -167,12 +152,6 @@ cudaError_t scsp_resident_nodes(int dims, int storage, uint32_t* nodes)
 {
     return dims == 3 ? resident_storage<D3Q19>(storage, nullptr, nullptr, nodes)
                      : resident_storage<D2Q9>(storage, nullptr, nullptr, nodes);
-}
-
-void launch_scsp_zou_he(int dims, int storage, const ScspLaunch& a, const ZouHe& z)
-{
-    if (dims == 3) zou_he_storage<D3Q19>(storage, a, z);
-    else zou_he_storage<D2Q9>(storage, a, z);
 }
 
 void launch_scsp_init(int dims, int storage, const Grid& g, const Force& F, double rho0,
