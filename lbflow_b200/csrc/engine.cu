@@ -32,6 +32,8 @@ struct lbf_engine {
     int cur = 0;
     uint2* occ = nullptr;
     uint32_t* coord = nullptr;
+    uint4 *link_row = nullptr, *link_base = nullptr;   // table of pull sources
+    uint32_t* link_mask = nullptr;
     uint8_t* node_label = nullptr;
     uint8_t* node_phase = nullptr;
     double* label_force = nullptr;
@@ -254,7 +256,7 @@ void launch_step(lbf_engine* e, bool pull, int out)
         e->sp.seed = dither && pull ? (++e->steps * 2654435761u) | 1u : 0u;
         e->sp.reverse = pull ? (int)(++e->pulls & 1u) : 0;
         ScspLaunch a{grid_of(e), e->force, e->sp, fin, fout, macros_of(e), e->err, e->stream,
-                     e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh};
+                     e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, Links{e->link_row, e->link_mask, e->link_base}};
         launch_scsp(e->D, (int)e->cfg.storage, e->cfg.collision == LBF_MRT, pull, out, a);
     } else {
         // 16-bit storage rounds stochastically with a fresh seed every pull
@@ -923,6 +925,29 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
                                                    e->coord, e->node_label, e->node_phase);
     LBF_CUDA(cudaGetLastError());
     LBF_CUDA(cudaMemcpyAsync(e->label_force, lforce.data(), lforce.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream));
+    if (c.model == LBF_MODEL_SCSP && scsp_uses_links(e->D, (int)c.storage)) {
+        const size_t tiles = (count + kLinkTile - 1) / kLinkTile;
+        LBF_ALLOC(e->link_row, tiles * kLinkTile);
+        LBF_ALLOC(e->link_mask, tiles * kLinkTile);
+        LBF_ALLOC(e->link_base, 2 * tiles);
+        // d_used has been read: its first word counts the nodes without offsets.
+        LBF_CUDA(cudaMemsetAsync(d_used, 0, sizeof(uint32_t), e->stream));
+        launch_build_links(grid_of(e), e->link_row, e->link_mask, e->link_base, d_used, e->stream);
+        LBF_CUDA(cudaGetLastError());
+        uint32_t none = 0;
+        LBF_CUDA(cudaMemcpyAsync(e->h_red, d_used, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
+        LBF_CUDA(cudaStreamSynchronize(e->stream));
+        std::memcpy(&none, e->h_red, sizeof none);
+        // Planes of more than about 65,000 fluid nodes overflow everywhere: the
+        // lookups alone are then the faster form.
+        if (none > e->nf / 16) {
+            cudaFreeAsync(e->link_row, e->stream);
+            cudaFreeAsync(e->link_mask, e->stream);
+            cudaFreeAsync(e->link_base, e->stream);
+            e->link_row = e->link_base = nullptr;
+            e->link_mask = nullptr;
+        }
+    }
     if (boundaries || c.model == LBF_MODEL_COLOR) {
         if ((rc = ensure_vox(e))) { std::string m = e->last_error; lbf_destroy(e); return fail(nullptr, rc, m); }
     }
@@ -1116,7 +1141,8 @@ void lbf_destroy(lbf_engine* e)
                     e->rho0, e->rho1, e->u, e->uprev, e->uadj, e->ind, e->indprev, e->indadj,
                     e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red,
                     e->zh_node, e->zh_code, e->zh_bits, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
-                    e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words};
+                    e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words,
+                    e->link_row, e->link_mask, e->link_base};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, e->stream);
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->h_red) cudaFreeHost(e->h_red);
@@ -1323,7 +1349,7 @@ bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
     const bool dither = e->cfg.storage == LBF_STORE_FP16 || e->cfg.storage == LBF_STORE_BF16;
     e->sp.seed = dither ? e->steps + 1 : 0;
     const ScspLaunch a{grid_of(e), e->force, e->sp, e->f[e->cur], e->f[e->cur ^ 1], macros_of(e), e->err, e->stream,
-                       e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh};
+                       e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, Links{e->link_row, e->link_mask, e->link_base}};
     if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess) {
         cudaGetLastError();
         e->resident_nodes = 0;

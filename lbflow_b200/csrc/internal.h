@@ -22,6 +22,7 @@ struct ScspLaunch {
     int8_t* eout;
     int out;             // kOutMacros / kOutAdjacent of this step
     ZouHe zh;            // PB/VB boundary nodes (n = 0: none)
+    Links links;         // table of pull sources (row = nullptr: none)
 };
 
 struct ColorLaunch {
@@ -42,6 +43,9 @@ struct ColorLaunch {
 
 // storage: LBF_STORE_* value; dims: 2 or 3.
 void launch_scsp(int dims, int storage, bool mrt, bool pull, int out, const ScspLaunch& a);
+// The table of pull sources: whether a storage's steps use it, and its fill.
+bool scsp_uses_links(int dims, int storage);
+void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, uint32_t* none, cudaStream_t s);
 void launch_scsp_init(int dims, int storage, const Grid& g, const Force& F, double rho0,
                       void* f, int8_t* eout, cudaStream_t s);
 // All steps of a call in one launch (resident.cuh): a.out applies to the last.

@@ -349,11 +349,125 @@ __device__ __forceinline__ uint32_t pull_sources(const Grid& g, int x, int y, in
     return mask;
 }
 
-template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4)>
+// ---- pull sources from a table ------------------------------------------------
+// The 16-bit storages' steps are bound by instruction issue, and the table
+// saves a seventh of their instructions (FP16: 802 -> 692 per node; 256^3
+// 110.3 -> 100.0 us per step, 192^3 47.9 -> 44.7; BFP16 192^3 55.6 -> 51.5).
+// Wider populations are bound by memory and lose by its 16 bytes per node
+// (FP32 256^3 110.9 -> 112.2, FP64 182 -> 216, where it also spills): they
+// keep the lookups.  For D3Q19 the sources lie in the node's own x-row
+// and eight others, and a row's three sources follow from the compact index of
+// its voxel at x: one less, itself, or itself plus its fluid bit.  The table
+// keeps that index for the eight rows as 16-bit offsets from a per-tile base
+// (tiles of 128 consecutive nodes, the step kernel's blocks), and a word with
+// the 18 fluid bits and two marks for x = 0 and x = nx - 1, whose sources
+// beyond the wrap are looked up as before: 20 bytes per node in place of the
+// 4-byte coordinate.  A third mark sends a node to the lookups altogether:
+// one whose offsets do not fit (a tile across the end of the first or last
+// plane, whose z neighbours wrap).
+struct Links {
+    const uint4* __restrict__ row;       // [node] eight 16-bit offsets
+    const uint32_t* __restrict__ mask;   // [node] bit q: the source of q is fluid
+    const uint4* __restrict__ base;      // [tile][2] bases of the eight rows
+};
+constexpr uint32_t kLinkTile = 128;
+constexpr uint32_t kLinkLeft = 1u << 30, kLinkRight = 1u << 31;   // mask marks: x = 0, x = nx - 1
+constexpr uint32_t kLinkNone = 1u << 29;                          // ... and no offsets
+
+// Row number of the sources at (y + dy, z + dz), and the direction pulling
+// from (x, y + dy, z + dz).
+__host__ __device__ constexpr int link_row(int dy, int dz)
+{
+    return dz == 0 ? (dy < 0 ? 0 : 1) : (dy == 0 ? (dz < 0 ? 2 : 3) : (dy < 0 ? (dz < 0 ? 4 : 5) : (dz < 0 ? 6 : 7)));
+}
+__host__ __device__ constexpr int link_dy(int r) { return r == 0 || r == 4 || r == 5 ? -1 : (r == 2 || r == 3 ? 0 : 1); }
+__host__ __device__ constexpr int link_dz(int r) { return r < 2 ? 0 : (r == 2 || r == 4 || r == 6 ? -1 : 1); }
+template <class L> __host__ __device__ constexpr int link_centre(int r)
+{
+    for (int q = 1; q < L::Q; ++q)
+        if (L::ex(q) == 0 && L::ey(q) == -link_dy(r) && L::ez(q) == -link_dz(r)) return q;
+    return 0;
+}
+
+template <class L>
+__device__ __forceinline__ uint32_t link_sources(const Grid& g, const Links& k, const uint32_t i, uint32_t (&src)[L::Q])
+{
+    const uint4 d = __ldg(&k.row[i]);
+    const uint32_t m = __ldg(&k.mask[i]);
+    const uint4 b0 = __ldg(&k.base[2 * (i / kLinkTile)]), b1 = __ldg(&k.base[2 * (i / kLinkTile) + 1]);
+    const uint32_t row[8] = {b0.x + (d.x & 0xffffu), b0.y + (d.x >> 16), b0.z + (d.y & 0xffffu), b0.w + (d.y >> 16),
+                             b1.x + (d.z & 0xffffu), b1.y + (d.z >> 16), b1.z + (d.w & 0xffffu), b1.w + (d.w >> 16)};
+#pragma unroll
+    for (int q = 1; q < L::Q; ++q) {
+        if (L::ey(q) == 0 && L::ez(q) == 0) src[q] = L::ex(q) > 0 ? i - 1 : i + 1;
+        else {
+            const int r = link_row(-L::ey(q), -L::ez(q));
+            src[q] = L::ex(q) == 0 ? row[r] : (L::ex(q) > 0 ? row[r] - 1 : row[r] + ((m >> link_centre<L>(r)) & 1u));
+        }
+    }
+    if (m & (kLinkLeft | kLinkRight | kLinkNone)) {
+        int x, y, z;
+        unpack(__ldg(&g.coord[i]), x, y, z);
+        if (m & kLinkNone) return pull_sources<L, true>(g, x, y, z, src);
+#pragma unroll
+        for (int q = 1; q < L::Q; ++q) {
+            if (L::ex(q) == 0) continue;
+            if (m & (L::ex(q) > 0 ? kLinkLeft : kLinkRight)) {
+                bool fluid;
+                src[q] = lookup(g, wrap(x - L::ex(q), g.nx), wrap(y - L::ey(q), g.ny), wrap(z - L::ez(q), g.nz), fluid);
+            }
+        }
+    }
+    return m;
+}
+
+// Fills the table, one block per tile; *none counts the nodes without offsets.
+template <class L>
+__global__ void __launch_bounds__(kLinkTile)
+build_links(const Grid g, uint4* __restrict__ row, uint32_t* __restrict__ mask, uint4* __restrict__ base,
+            uint32_t* __restrict__ none)
+{
+    __shared__ uint32_t low[8];
+    const uint32_t i = blockIdx.x * kLinkTile + threadIdx.x;
+    if (threadIdx.x < 8) low[threadIdx.x] = 0xffffffffu;
+    __syncthreads();
+    uint32_t idx[8] = {0, 0, 0, 0, 0, 0, 0, 0}, m = 0;
+    if (i < g.nf) {
+        int x, y, z;
+        unpack(g.coord[i], x, y, z);
+        uint32_t src[L::Q];
+        m = pull_sources<L, true>(g, x, y, z, src) | (x == 0 ? kLinkLeft : 0u) | (x + 1 == g.nx ? kLinkRight : 0u);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            idx[r] = src[link_centre<L>(r)];
+            atomicMin(&low[r], idx[r]);
+        }
+    }
+    __syncthreads();
+    if (i < g.nf) {
+        uint32_t d[8], worst = 0;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) { d[r] = idx[r] - low[r]; worst |= d[r]; }
+        if (worst > 0xffffu) {
+            atomicAdd(none, 1u);
+            m |= kLinkNone;
+        }
+        row[i] = make_uint4((d[0] & 0xffffu) | (d[1] << 16), (d[2] & 0xffffu) | (d[3] << 16),
+                            (d[4] & 0xffffu) | (d[5] << 16), (d[6] & 0xffffu) | (d[7] << 16));
+        mask[i] = m;
+    }
+    if (threadIdx.x < 2) {
+        const uint32_t* l = low + 4 * threadIdx.x;
+        base[2 * blockIdx.x + threadIdx.x] = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+}
+
+template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4), bool LINKS = false>
 __device__ __forceinline__ void gather(const Grid& g, const typename S::T* __restrict__ fin,
                                        uint32_t i, int x, int y, int z,
                                        typename S::R (&f)[L::Q], uint32_t (&nbr)[L::Q],
-                                       typename S::R rho0, const int8_t* __restrict__ ein = nullptr)
+                                       typename S::R rho0, const int8_t* __restrict__ ein = nullptr,
+                                       const Links& links = Links{})
 {
     // Element offsets stay 32-bit (phases * Q * nfp < 2^32 is checked at
     // creation); only the final address is 64-bit.
@@ -367,7 +481,9 @@ __device__ __forceinline__ void gather(const Grid& g, const typename S::T* __res
         return;
     }
     uint32_t src[L::Q];
-    const uint32_t mask = pull_sources<L, UNIFORM>(g, x, y, z, src);
+    uint32_t mask;
+    if constexpr (LINKS) mask = link_sources<L>(g, links, i, src);
+    else mask = pull_sources<L, UNIFORM>(g, x, y, z, src);
     pdl_wait();
     f[0] = load_pop<S>(fin + i, 0, rho0, ein, i);
 #pragma unroll
@@ -611,18 +727,19 @@ __device__ __forceinline__ void scsp_store(const Grid& g, const ScspParams& P, t
 
 // Update of one fluid node i (the body of scsp_step, shared with the batched
 // kernel).
-template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4)>
+template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4), bool LINKS = false>
 __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const ScspParams& P,
                                             const typename S::T* __restrict__ fin,
                                             typename S::T* __restrict__ fout, const uint32_t i,
                                             const Macros& mo, const int out, uint32_t* __restrict__ err,
-                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout,
+                                            const Links& links = Links{})
 {
-    int x, y, z;
-    unpack(__ldg(&g.coord[i]), x, y, z);
+    int x = 0, y = 0, z = 0;
+    if (!LINKS) unpack(__ldg(&g.coord[i]), x, y, z);
     typename S::R f[L::Q];
     uint32_t nbr[L::Q];
-    gather<L, S, PULL, UNIFORM>(g, fin, i, x, y, z, f, nbr, typename S::R(P.rho0), ein);
+    gather<L, S, PULL, UNIFORM, LINKS>(g, fin, i, x, y, z, f, nbr, typename S::R(P.rho0), ein, links);
     scsp_collide<L, S>(g, F, P, i, f, mo, out, err);
     scsp_store<L, S>(g, P, fout, i, f, eout);
 }
@@ -740,9 +857,9 @@ __device__ __forceinline__ typename S::R zou_he_node(typename S::R (&f)[L::Q], u
 // Update of the k-th boundary node.
 template <class L, class S>
 __device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, const ZouHe& z, const uint32_t k,
-                                            const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-                                            const Macros& mo, const int out, uint32_t* __restrict__ err,
-                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+                                         const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+                                         const Macros& mo, const int out, uint32_t* __restrict__ err,
+                                         const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
 {
     using R = typename S::R;
     const uint32_t i = __ldg(&z.node[k]);
@@ -837,12 +954,13 @@ __device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, 
 
 // One step of every node.  BOUNDARY: the grid's first `zblocks` blocks update
 // the Zou-He nodes and the others leave them out.
-template <class L, class S, bool PULL, bool BOUNDARY>
+template <class L, class S, bool PULL, bool BOUNDARY, bool LINKS>
 __global__ void __launch_bounds__(128, BOUNDARY ? StepBlocks<S>::boundary : StepBlocks<S>::value)
 scsp_step(const Grid g, const Force F, const ScspParams P,
           const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
           Macros mo, const int out, uint32_t* __restrict__ err,
-          const int8_t* __restrict__ ein, int8_t* __restrict__ eout, const ZouHe z, const uint32_t zblocks)
+          const int8_t* __restrict__ ein, int8_t* __restrict__ eout, const ZouHe z, const uint32_t zblocks,
+          const Links links)
 {
     // The node order alternates between steps: a step that runs in the
     // opposite order to the previous one starts with the nodes whose
@@ -861,7 +979,7 @@ scsp_step(const Grid g, const Force F, const ScspParams P,
     const uint32_t i = (P.reverse ? blocks - 1 - b : b) * blockDim.x + threadIdx.x;
     if (i >= g.nf) return;
     if (BOUNDARY && ((__ldg(&z.bits[i >> 5]) >> (i & 31)) & 1u)) return;
-    scsp_update<L, S, PULL>(g, F, P, fin, fout, i, mo, out, err, ein, eout);
+    scsp_update<L, S, PULL, (sizeof(typename S::R) == 4), LINKS>(g, F, P, fin, fout, i, mo, out, err, ein, eout, links);
 }
 
 // t = 0 populations of SCSP::initialize (scsp.cpp:116-134):

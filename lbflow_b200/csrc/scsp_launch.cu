@@ -5,6 +5,11 @@
 namespace lbf {
 
 namespace {
+// Which steps take their sources from the table: 16-bit storage (see Links).
+template <class L, class S> struct UseLinks {
+    static constexpr bool value = L::D == 3 && sizeof(typename S::T) == 2;
+};
+
 template <class L, class S>
 void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
 {
@@ -17,15 +22,24 @@ void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
     // At t = 0 (no pull) the boundary nodes hold rho0 at rest, which the
     // ordinary update reproduces from their initial populations.
     const unsigned zb = pull ? blocks_for(a.zh.n, threads) : 0;
-    if (zb)
-        launch_pdl(scsp_step<L, S, true, true>, zb + blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out,
-                   a.err, a.ein, a.eout, a.zh, zb);
-    else if (pull)
-        launch_pdl(scsp_step<L, S, true, false>, blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err,
-                   a.ein, a.eout, a.zh, 0u);
-    else
-        scsp_step<L, S, false, false><<<blocks, threads, 0, a.stream>>>(a.g, a.F, a.P, fin, fout, a.mo, out, a.err,
-                                                                        a.ein, a.eout, a.zh, 0u);
+    auto step = [&](auto kernel) {
+        launch_pdl(kernel, zb + blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout,
+                   a.zh, zb, a.links);
+    };
+    if (!pull) {
+        scsp_step<L, S, false, false, false><<<blocks, threads, 0, a.stream>>>(
+            a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout, a.zh, 0u, a.links);
+        return;
+    }
+    if constexpr (UseLinks<L, S>::value) {
+        if (a.links.row) {
+            if (zb) step(scsp_step<L, S, true, true, true>);
+            else step(scsp_step<L, S, true, false, true>);
+            return;
+        }
+    }
+    if (zb) step(scsp_step<L, S, true, true, false>);
+    else step(scsp_step<L, S, true, false, false>);
 }
 
 template <class L>
@@ -122,6 +136,17 @@ void add_density_storage(int storage, const Grid& g, const float* drho, void* f,
     }
 }
 }  // namespace
+
+bool scsp_uses_links(int dims, int storage)
+{
+    return dims == 3 && storage != LBF_STORE_FP64 && storage != LBF_STORE_FP32;
+}
+
+void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, uint32_t* none, cudaStream_t s)
+{
+    const unsigned blocks = blocks_for(g.nf, kLinkTile);
+    if (blocks) build_links<D3Q19><<<blocks, kLinkTile, 0, s>>>(g, row, mask, base, none);
+}
 
 void launch_scsp_add_density(int dims, int storage, const Grid& g, const float* drho, void* f, int8_t* e,
                              double rho0, cudaStream_t s)
