@@ -333,6 +333,32 @@ struct IgemmLoader {
     __device__ uint64_t bdesc(int s, int kk) const { return desc_sw128(r.b(s) + 32u * kk, 16u, 1024u); }
 };
 
+// Bias of 16 accumulator columns from nb, bias entries from `from` on, wrapping
+// at p.ld in the scatter mode.  One branch for all 16: with one per column
+// (bias or not, activation or not) these were the slowest part of the
+// epilogue, 84 cycles a column.
+__device__ __forceinline__ void add_bias(const IgemmArgs& p, float (&v)[16], uint32_t nb, uint32_t from) {
+    if (!p.bias) return;
+    const uint32_t period = p.mode == LBF_OUT_SCATTER2_BF16 ? p.ld : 0xffffffffu;
+    float b[16];
+#pragma unroll
+    for (uint32_t e = 0; e < 16u; ++e) {
+        b[e] = nb + e < p.n ? __ldg(p.bias + from) : 0.f;
+        from = from + 1u == period ? 0u : from + 1u;
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) v[e] += b[e];
+}
+
+__device__ __forceinline__ void st_shared16(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared16(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+
 template <int BN>
 __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constant__ IgemmArgs p) {
     extern __shared__ uint8_t smem_raw[];
@@ -353,20 +379,16 @@ __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constan
     const uint32_t row = m0 + warp * 32 + lane;
     const bool rvalid = ok && row < p.g.rows;
     Coord rc = row_coord(p.g, rvalid ? row : 0u);
+    const float slope = p.act ? p.slope : 1.f;
 #pragma unroll 1
     for (int col0 = 0; col0 < BN; col0 += 16) {
         float v[16];
         tmem_ld16(tmem + ((warp * 32u) << 16) + uint32_t(col0), v);
         if (!rvalid) continue;
         const uint32_t nb = n0 + col0;
+        add_bias(p, v, nb, p.mode == LBF_OUT_SCATTER2_BF16 ? nb % p.ld : nb);
 #pragma unroll
-        for (int e = 0; e < 16; ++e) {
-            const uint32_t n = nb + e;
-            float x = v[e];
-            if (p.bias && n < p.n) x += p.bias[p.mode == LBF_OUT_SCATTER2_BF16 ? n % p.ld : n];
-            if (p.act) x = x > 0.f ? x : x * p.slope;
-            v[e] = x;
-        }
+        for (int e = 0; e < 16; ++e) v[e] = v[e] > 0.f ? v[e] : v[e] * slope;
         if (p.mode == LBF_OUT_F32) {
             float* o = static_cast<float*>(p.out) + size_t(row) * p.ld;
             for (int e = 0; e < 16; ++e)
@@ -417,6 +439,228 @@ __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constan
                 __nv_bfloat16 h = __float2bfloat16_rn(v[e]);
                 o[c + e] = *reinterpret_cast<uint16_t*>(&h);
             }
+        }
+    }
+    release(tmem, kCols);
+}
+
+// ---------------------------------------------------------------- conv3 ----
+
+// Periodic 3x3x3 convolution of up to 64 channels from a tile with halo in
+// shared memory.  igemm gathers the 27 taps of a row separately, so every
+// input voxel crosses from L2 27 times, and with fewer than 64 channels its
+// producers spend their time on tap arithmetic.  Here a block computes
+// 8 (x) x 16 (y) x kCZ (z) outputs: it copies the 10 x 18 x (kCZ + 2) input
+// voxels once, as 16-byte pieces [8 channels][voxel], which is the unswizzled
+// K-major operand layout: 8 voxels along x are a core matrix, the 16 rows
+// along y follow at the tile's row pitch, and a tap is a start address
+// (dz, dy, dx) voxels further on.  The weights [tap][8 channels][n] stay in
+// shared memory where they are few, else they stream through a ring of `stages`
+// slots of `per` taps (a slot per tap is bound by the latency of its refill);
+// each is used by the kCZ z slices' accumulators.  The K order per output is
+// igemm's (tap, then channel).
+//
+// Measured, igemm -> here: 16 -> 16 channels at 96^3 238 -> 61 us, 32 -> 16
+// (two sources) 403 -> 104, 32 -> 32 at 48^3 63 -> 22, 64 -> 64 at 2 x 48^3
+// 91 -> 82.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
+// (cp.async at 14 bytes a cycle), 28,000 for 432 MMAs (N = 64, 65 cycles each;
+// operand reads alone need 48), the rest weights and epilogue.  8 producer
+// warps: 16 take 96 us for 16 -> 16, their registers cost a resident block.
+constexpr int kCX = 8, kCY = 16, kCZ = 4;
+constexpr int kHX = kCX + 2, kHY = kCY + 2, kHZ = kCZ + 2;
+constexpr int kHalo = kHX * kHY * kHZ;
+// Channel groups' planes are one piece longer than the tile: the copies of a
+// voxel's consecutive groups then fall into different banks.
+constexpr uint32_t kPlane = (kHalo + 1) * 16;
+constexpr int kTapStages = 3;      // most slots
+constexpr int kConvProducers = 256, kConvThreads = kConvProducers + 32;
+constexpr uint32_t kMaxConvC = 64;
+struct TapRing { uint32_t per, stages; };
+
+constexpr size_t conv3_smem(uint32_t groups, uint32_t bn, TapRing r) {
+    return 128 + size_t(groups) * kPlane + size_t(r.per) * r.stages * groups * bn * 16 + (2 + 2 * kTapStages) * 8 + 16;
+}
+
+// G: 8-channel groups held (2, 4 or 8; those past the input's channels are
+// zeros).
+template <int BN, int G>
+__global__ void __launch_bounds__(kConvThreads, 1)
+conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint32_t ty, const uint32_t tz,
+             const TapRing ring) {
+    extern __shared__ uint8_t smem_raw[];
+    constexpr uint32_t kCols = kCZ * BN;
+    constexpr uint32_t tap_bytes = G * BN * 16u;
+    const uint32_t a0 = (smem_u32(smem_raw) + 127u) & ~127u;
+    const uint32_t w0 = a0 + G * kPlane;
+    const uint32_t slot_bytes = ring.per * tap_bytes;
+    const uint32_t bar = (w0 + ring.stages * slot_bytes + 7u) & ~7u;
+    const uint32_t full_a = bar, done = bar + 8u, full0 = bar + 16u, empty0 = full0 + kTapStages * 8u;
+    const uint32_t slot = empty0 + kTapStages * 8u;
+
+    if (threadIdx.x < 32) {
+        tmem_alloc(slot, kCols);
+        tmem_relinquish();
+    }
+    if (threadIdx.x == 0) {
+        mbar_init(full_a, kConvProducers);
+        mbar_init(done, 1);
+        for (int s = 0; s < kTapStages; ++s) {
+            mbar_init(full0 + 8u * s, kConvProducers);
+            mbar_init(empty0 + 8u * s, 1);
+        }
+        mbar_init_fence();
+    }
+    fence_before_sync();
+    __syncthreads();
+    fence_after_sync();
+    uint32_t tmem;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(slot) : "memory");
+    tmem = __shfl_sync(0xffffffffu, tmem, 0);
+
+    uint32_t t = blockIdx.x;
+    const int x0 = int(t % tx) * kCX;
+    t /= tx;
+    const int y0 = int(t % ty) * kCY;
+    t /= ty;
+    const int z0 = int(t % tz) * kCZ;
+    const uint32_t b = t / tz;
+    const uint32_t n0 = blockIdx.y * BN;
+    const uint32_t warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+
+    bool ok = true;
+    if (warp < uint32_t(kConvProducers / 32)) {
+        // A thread copies one group of the 10 voxels of a tile row at a time, the
+        // threads of consecutive groups side by side; its x offsets are the same
+        // in every row.  Voxels past the grid belong to no valid output: any
+        // address will do.
+        constexpr uint32_t kStep = kConvProducers / G;
+        auto inside = [](int v, int n) {
+            v = wrap(v, n);
+            return v < n ? v : 0;
+        };
+        const uint32_t g8 = threadIdx.x % G, first = threadIdx.x / G, ch = g8 * 8u;
+        const bool in = ch < p.g.ct;
+        const uint32_t c = ch < p.g.c0 ? p.g.c0 : p.g.c1;
+        const uint16_t* const src = !in ? p.g.src0 : (ch < p.g.c0 ? p.g.src0 + ch : p.g.src1 + (ch - p.g.c0));
+        const uint32_t bytes = in ? 16u : 0u;
+        uint32_t xo[kHX];
+#pragma unroll
+        for (int i = 0; i < kHX; ++i) xo[i] = in ? uint32_t(inside(x0 + i - 1, int(p.g.in_w))) * c : 0u;
+        for (uint32_t r = first; r < kHY * kHZ; r += kStep) {
+            const uint32_t hz = r / kHY, hy = r - hz * kHY;
+            const int z = inside(z0 + int(hz) - 1, int(p.g.in_d)), y = inside(y0 + int(hy) - 1, int(p.g.in_h));
+            const size_t vox = ((size_t(b) * p.g.in_d + z) * p.g.in_h + y) * p.g.in_w;
+            const uint16_t* const row = in ? src + vox * c : src;
+            const uint32_t dst = a0 + g8 * kPlane + r * (kHX * 16u);
+#pragma unroll
+            for (int i = 0; i < kHX; ++i) cp_async16(dst + i * 16u, row + xo[i], bytes);
+        }
+        cp_async_arrive(full_a);
+        const uint16_t* const wp = in ? p.w + size_t(n0) * p.k_pad + ch : p.w;
+        const uint32_t total = 27u / ring.per;
+        for (uint32_t st = 0; st < total; ++st) {
+            const uint32_t s = st % ring.stages;
+            if (st >= ring.stages) {
+                const bool w = mbar_wait(empty0 + 8u * s, (st / ring.stages - 1u) & 1u, kWaitCycles);
+                ok = __all_sync(0xffffffffu, w);
+                if (!ok) break;
+            }
+            for (uint32_t q = first; q < ring.per * BN; q += kStep) {
+                const uint32_t tap = q / BN, n = q % BN;
+                cp_async16(w0 + s * slot_bytes + tap * tap_bytes + (g8 * BN + n) * 16u,
+                           in ? wp + n * p.k_pad + (st * ring.per + tap) * p.g.ct : wp, bytes);
+            }
+            cp_async_arrive(full0 + 8u * s);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        const bool d = mbar_wait(done, 0u, kWaitCycles);
+        fence_after_sync();
+        ok = ok && d;
+    } else {
+        // The whole warp, converged; one lane issues.
+        const uint32_t leader = elect_one();
+        constexpr uint32_t idesc = idesc_bf16(kBM, BN, false, false);
+        bool go = __all_sync(0xffffffffu, mbar_wait(full_a, 0u, kWaitCycles));
+        // Descriptors differ in their start address (16-byte units) only.
+        const uint64_t ad0 = desc_plain(a0, kPlane, kHX * 16u);
+        const uint64_t bd0 = desc_plain(w0, BN * 16u, 128u);
+        for (uint32_t st = 0; st < 27u / ring.per && go; ++st) {
+            const uint32_t s = st % ring.stages;
+            go = __all_sync(0xffffffffu, mbar_wait(full0 + 8u * s, (st / ring.stages) & 1u, kWaitCycles));
+            if (!go) break;
+            fence_async_shared();
+            fence_after_sync();
+            for (uint32_t j = 0; j < ring.per; ++j) {
+                const uint32_t tap = st * ring.per + j;
+                const uint32_t dz = tap / 9u, dy = tap / 3u - 3u * dz, dx = tap % 3u;
+                uint64_t ad = ad0 + (dz * kHY + dy) * kHX + dx;
+                uint64_t bd = bd0 + (s * slot_bytes + j * tap_bytes) / 16u;
+                for (uint32_t k = 0; k < uint32_t(G); k += 2, ad += 2 * kPlane / 16u, bd += 2 * BN)
+#pragma unroll
+                    for (uint32_t z = 0; z < uint32_t(kCZ); ++z)
+                        mma_bf16_warp(leader, tmem + z * BN, ad + z * (kHX * kHY), bd, idesc, (tap | k) != 0u);
+            }
+            commit_warp(leader, empty0 + 8u * s);
+        }
+        commit_warp(leader, done);
+    }
+    if (warp >= uint32_t(kConvProducers / 32)) {
+        release(tmem, kCols);
+        return;
+    }
+    if (!ok && threadIdx.x == 0) atomicOr(p.err, LBF_ERR_MMA_TIMEOUT);
+
+    // Accumulator row 8 y + x of each z slice; warp w reads lanes 32 (w mod 4)
+    // on, four warps every other slice.
+    const uint32_t quarter = warp & 3u, m = quarter * 32u + lane;
+    const uint32_t x = uint32_t(x0) + (m & 7u), y = uint32_t(y0) + (m >> 3);
+    // Rows that allow 16-byte bf16 stores go through shared memory (the tile is
+    // no longer read): lanes then store consecutive pieces of the 8 voxels of a
+    // tile row, one run in memory.
+    const bool vec = p.mode == LBF_OUT_BF16 && p.ld % 8u == 0u && p.n % 8u == 0u;
+    const float slope = p.act ? p.slope : 1.f;
+    constexpr uint32_t kPitch = BN * 2u + 16u, kParts = BN / 8u;
+    const uint32_t stage = a0 + warp * 32u * kPitch;
+#pragma unroll 1
+    for (uint32_t zi = warp >> 2; zi < uint32_t(kCZ); zi += kConvProducers / 128) {
+        const uint32_t z = uint32_t(z0) + zi;
+        const bool valid = ok && x < p.g.out_w && y < p.g.out_h && z < p.g.out_d;
+        const size_t row = ((size_t(b) * p.g.out_d + z) * p.g.out_h + y) * p.g.out_w + x;
+#pragma unroll 1
+        for (uint32_t col0 = 0; col0 < uint32_t(BN); col0 += 16u) {
+            float v[16];
+            tmem_ld16(tmem + ((quarter * 32u) << 16) + zi * BN + col0, v);
+            const uint32_t nb = n0 + col0;
+            add_bias(p, v, nb, nb);
+#pragma unroll
+            for (uint32_t e = 0; e < 16u; ++e) v[e] = v[e] > 0.f ? v[e] : v[e] * slope;
+            if (vec) {
+                const uint32_t at = stage + lane * kPitch + col0 * 2u;
+                st_shared16(at, pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                st_shared16(at + 16u, pack_bf16(v[8], v[9]), pack_bf16(v[10], v[11]), pack_bf16(v[12], v[13]),
+                            pack_bf16(v[14], v[15]));
+            } else if (valid) {
+#pragma unroll
+                for (uint32_t e = 0; e < 16u; ++e) {
+                    if (nb + e >= p.n) continue;
+                    if (p.mode == LBF_OUT_F32) static_cast<float*>(p.out)[row * p.ld + nb + e] = v[e];
+                    else static_cast<__nv_bfloat16*>(p.out)[row * p.ld + nb + e] = __float2bfloat16_rn(v[e]);
+                }
+            }
+        }
+        if (vec) {
+            __syncwarp();
+            for (uint32_t k = lane; k < 32u * kParts; k += 32u) {
+                const uint32_t r = k / kParts, part = k % kParts;
+                const uint32_t mr = quarter * 32u + r, xr = uint32_t(x0) + (mr & 7u), yr = uint32_t(y0) + (mr >> 3);
+                const uint32_t n = n0 + part * 8u;
+                if (!ok || xr >= p.g.out_w || yr >= p.g.out_h || z >= p.g.out_d || n >= p.n) continue;
+                const size_t vox = ((size_t(b) * p.g.out_d + z) * p.g.out_h + yr) * p.g.out_w + xr;
+                *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + vox * p.ld + n) =
+                    ld_shared16(stage + r * kPitch + part * 16u);
+            }
+            __syncwarp();
         }
     }
     release(tmem, kCols);
@@ -656,6 +900,44 @@ int launch_igemm(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
     return LBF_OK;
 }
 
+// Whether conv3_kernel takes the call: a 3x3x3 periodic convolution of at most
+// kMaxConvC channels into rows, whose tiles are not mostly padding.
+bool conv3_fits(const IgemmArgs& p) {
+    const Gather& g = p.g;
+    if (g.ks != 3 || g.stride != 1 || g.pad != 1 || g.ct > kMaxConvC || p.mode == LBF_OUT_SCATTER2_BF16 ||
+        g.in_d != g.out_d || g.in_h != g.out_h || g.in_w != g.out_w)
+        return false;
+    auto up = [](uint64_t n, uint64_t t) { return (n + t - 1) / t * t; };
+    return up(g.out_w, kCX) * up(g.out_h, kCY) * up(g.out_d, kCZ) <= 2ull * g.out_w * g.out_h * g.out_d;
+}
+
+constexpr int kSmemMost = 227 * 1024;     // shared memory of a block, and of an SM's blocks together
+
+template <int BN, int G>
+int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
+    // All 27 taps' weights where that leaves room for three blocks on an SM, else
+    // three slots of as many taps as fit into one block's shared memory.
+    TapRing ring{27, 1};
+    if (conv3_smem(G, BN, ring) > kSmemMost / 3) ring = TapRing{3, 3};
+    if (conv3_smem(G, BN, ring) > kSmemMost) ring = TapRing{1, 3};
+    const size_t sm = conv3_smem(G, BN, ring);
+    cudaError_t e = cudaFuncSetAttribute(conv3_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
+    if (e == cudaSuccess) {
+        const uint32_t tx = (p.g.out_w + kCX - 1) / kCX, ty = (p.g.out_h + kCY - 1) / kCY, tz = (p.g.out_d + kCZ - 1) / kCZ;
+        const uint32_t batch = p.g.rows / (p.g.out_w * p.g.out_h * p.g.out_d);
+        conv3_kernel<BN, G><<<dim3(tx * ty * tz * batch, n_pad / BN), kConvThreads, sm, s>>>(p, tx, ty, tz, ring);
+        e = cudaGetLastError();
+    }
+    if (e != cudaSuccess) return fail(std::string("lbf_igemm_run: ") + cudaGetErrorString(e), LBF_ECUDA);
+    return LBF_OK;
+}
+
+template <int BN>
+int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
+    return p.g.ct <= 16 ? launch_conv3<BN, 2>(p, n_pad, s)
+                        : (p.g.ct <= 32 ? launch_conv3<BN, 4>(p, n_pad, s) : launch_conv3<BN, 8>(p, n_pad, s));
+}
+
 struct WgradPlan {
     uint32_t bn, tiles_m, tiles_n, nch, cps, splits;
     size_t bytes;
@@ -710,6 +992,14 @@ int lbf_igemm_run(const lbf_igemm* d, void* stream) {
     p.slope = d->slope;
     p.err = d->err;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (conv3_fits(p)) {
+        switch (np) {
+            case 16: return launch_conv3<16>(p, np, s);
+            case 32: return launch_conv3<32>(p, np, s);
+            case 64: return launch_conv3<64>(p, np, s);
+            default: return launch_conv3<128>(p, np, s);
+        }
+    }
     switch (np) {
         case 16: return launch_igemm<16>(p, np, s);
         case 32: return launch_igemm<32>(p, np, s);

@@ -34,6 +34,18 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr, uint32_t lbo_byte
     return d;
 }
 
+// Unswizzled K-major operand: core matrices of 8 rows x 16 bytes, the rows of
+// one 16 bytes apart; `lbo` bytes between the core matrices along K, `sbo`
+// between those along M/N.  The start address needs 16-byte alignment only.
+__device__ __forceinline__ uint64_t desc_plain(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
+    uint64_t d = 0;
+    d |= static_cast<uint64_t>((saddr >> 4) & 0x3FFFu);
+    d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
+    d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
+    d |= static_cast<uint64_t>(1u) << 46;   // descriptor version for sm_100
+    return d;
+}
+
 // Instruction descriptor of kind::f16 with BF16 A/B and an F32 accumulator.
 __host__ __device__ constexpr uint32_t idesc_bf16(uint32_t M, uint32_t N, bool a_mn, bool b_mn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
@@ -47,6 +59,32 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t adesc, uint64
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
         :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u));
+}
+
+// One lane of a converged warp.
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(e));
+    return e;
+}
+
+// mma_bf16 and commit for a whole converged warp, issued by the lane with
+// `leader` set: with warp-uniform control flow the descriptors stay in uniform
+// registers.
+__device__ __forceinline__ void mma_bf16_warp(uint32_t leader, uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
+                                              uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, e;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 e, %6, 0;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}\n"
+        :: "r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0u), "r"(leader));
+}
+__device__ __forceinline__ void commit_warp(uint32_t leader, uint32_t mbar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+        :: "r"(mbar), "r"(leader) : "memory");
 }
 
 // Arrive once on an mbarrier when every tcgen05 operation issued so far by
