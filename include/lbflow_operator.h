@@ -87,6 +87,20 @@ typedef struct {
 size_t lbf_wgrad_workspace(const lbf_wgrad *w);
 int lbf_wgrad_run(const lbf_wgrad *w, void *stream);
 
+/* The weight matrix of lbf_igemm from an fp32 weight tensor: a 5-D view of it
+ * (element strides, negative ones allowed), whose first `split` dimensions
+ * make n and the others k, both row-major; bf16 [n_pad][k_pad], zero beyond.  */
+int lbf_pack_weight(const float *src, const uint32_t dims[5], const int64_t strides[5], uint32_t split, void *dst,
+                    uint32_t n_pad, uint32_t k_pad, void *stream);
+
+/* Backward of bias and leaky ReLU: out = gy * (y > 0 ? 1 : slope) rounded to
+ * bf16, and bias[c] = sum over rows of out (fp32, summed in a fixed order).
+ * gy, y, out: bf16 [rows][channels], 16-byte aligned; channels a multiple of
+ * 8, at most 2048.  y NULL: no activation, out unused, bias sums gy. */
+size_t lbf_act_grad_workspace(uint32_t channels);
+int lbf_act_grad(const void *gy, const void *y, float slope, uint64_t rows, uint32_t channels, void *out, float *bias,
+                 void *workspace, size_t workspace_bytes, void *stream);
+
 /* Compile-time facts of the kernels: tile rows, K per stage, stages. */
 void lbf_operator_info(uint32_t out[4]);
 

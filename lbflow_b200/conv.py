@@ -4,10 +4,11 @@ Functions (ctypes binding of include/lbflow_operator.h).
 Activations are channels-last bf16 tensors (batch, z, y, x, channel) whose
 channel counts are multiples of 8; weights are fp32 parameters in torch's
 layout, rounded to bf16 and packed into the kernels' K-major matrices at
-every call.  Forward convolutions, data gradients and weight gradients all
-run in the library's tcgen05 kernels; torch supplies device memory, the
-stream, the leaky-ReLU mask of the backward pass and bias sums.  There is no
-fallback: without the CUDA library every call raises.
+every call (one kernel).  Forward convolutions, data gradients and weight
+gradients all run in the library's tcgen05 kernels, the leaky-ReLU mask of
+the backward pass and the bias sums in one of its elementwise kernels; torch
+supplies device memory and the stream.  There is no fallback: without the
+CUDA library every call raises.
 
 Three operators:
   conv3  3x3x3 convolution with periodic wrap (one or two concatenated inputs)
@@ -15,6 +16,7 @@ Three operators:
   up2    2x2x2 transposed convolution with stride 2 (doubles the grid)
 """
 import ctypes
+import math
 
 import torch
 
@@ -56,6 +58,12 @@ def _lib():
         lib.lbf_wgrad_run.argtypes = [ctypes.POINTER(_Wgrad), P]
         lib.lbf_wgrad_workspace.restype = ctypes.c_size_t
         lib.lbf_wgrad_workspace.argtypes = [ctypes.POINTER(_Wgrad)]
+        lib.lbf_pack_weight.restype = ctypes.c_int
+        lib.lbf_pack_weight.argtypes = [P, ctypes.POINTER(U32), ctypes.POINTER(ctypes.c_int64), U32, P, U32, U32, P]
+        lib.lbf_act_grad_workspace.restype = ctypes.c_size_t
+        lib.lbf_act_grad_workspace.argtypes = [U32]
+        lib.lbf_act_grad.restype = ctypes.c_int
+        lib.lbf_act_grad.argtypes = [P, P, ctypes.c_float, ctypes.c_uint64, U32, P, P, P, ctypes.c_size_t, P]
         lib.lbf_operator_info.restype = None
         lib.lbf_operator_info.argtypes = [ctypes.POINTER(U32)]
         _SIGS = True
@@ -117,14 +125,50 @@ def pack_weight(mat):
     return out
 
 
+class _Packed:
+    """A packed weight matrix and its real extents."""
+
+    def __init__(self, data, n, k):
+        self.data, self.n, self.k = data, n, k
+
+
+def _pack(weight, order, split, flip=False):
+    """pack_weight of weight.permute(order) with its first `split` dimensions
+    as n and the others as k (flip: the kernel dimensions 2, 3, 4 reversed),
+    by one kernel straight from the parameter where it is an fp32 CUDA
+    tensor."""
+    if weight.dtype != torch.float32 or not weight.is_cuda:
+        w = (weight.flip(2, 3, 4) if flip else weight).permute(order)
+        n = math.prod(w.shape[:split])
+        mat = w.reshape(n, -1)
+        return _Packed(pack_weight(mat), *mat.shape)
+    dims = [weight.shape[d] for d in order]
+    strides = [weight.stride(d) for d in order]
+    at = weight.data_ptr()
+    if flip:
+        for j, d in enumerate(order):
+            if d >= 2:
+                at += 4 * strides[j] * (dims[j] - 1)
+                strides[j] = -strides[j]
+    n, k = math.prod(dims[:split]), math.prod(dims[split:])
+    out = torch.empty(_pad16(n), _pad64(k), dtype=torch.bfloat16, device=weight.device)
+    _ck(_lib().lbf_pack_weight(at, (U32 * 5)(*dims), (ctypes.c_int64 * 5)(*strides), split, out.data_ptr(),
+                               out.shape[0], out.shape[1], _stream(weight)))
+    return _Packed(out, n, k)
+
+
 def igemm(src0, src1, ksize, stride, pad, out_dims, wmat, bias=None, mode=OUT_BF16, out=None, out_ld=None,
           act=False, slope=0.0):
     """out[row][n] = act(sum_k A[row][k] wmat[n][k] + bias) on the tensor cores.
 
-    wmat: (n, k) with k = ksize^3 * channels (tap-major), any float dtype."""
+    wmat: (n, k) with k = ksize^3 * channels (tap-major), any float dtype, or
+    its packed form."""
     lib = _lib()
-    n, k = wmat.shape
-    wp = pack_weight(wmat)
+    if isinstance(wmat, _Packed):
+        wp, n, k = wmat.data, wmat.n, wmat.k
+    else:
+        n, k = wmat.shape
+        wp = pack_weight(wmat)
     g = _gather(src0, src1, ksize, stride, pad, out_dims)
     assert k == ksize ** 3 * (g.c0 + g.c1)
     B = src0.shape[0]
@@ -165,8 +209,28 @@ def wgrad(src0, src1, ksize, stride, pad, out_dims, b):
     return out
 
 
-def _lrelu_grad(gy, y, slope):
-    return (gy.float() * torch.where(y > 0, 1.0, slope)).to(torch.bfloat16).contiguous()
+def _act_grad(gy, y, slope, want_bias):
+    """(gradient before the activation as contiguous bf16, bias gradient or
+    None) of the incoming gradient gy; slope None: no activation."""
+    c = gy.shape[-1]
+    if gy.dtype == torch.bfloat16 and gy.is_cuda and gy.numel() and c % 8 == 0 and c <= 2048:
+        lib = _lib()
+        gy = gy.contiguous()
+        if gy.data_ptr() % 16:
+            gy = gy.clone()
+        out = torch.empty_like(gy) if slope is not None else gy
+        if slope is not None or want_bias:
+            gb = torch.empty(c, dtype=torch.float32, device=gy.device)
+            nbytes = lib.lbf_act_grad_workspace(c)
+            ws = torch.empty(nbytes // 4, dtype=torch.float32, device=gy.device)
+            _ck(lib.lbf_act_grad(gy.data_ptr(), y.data_ptr() if slope is not None else None, float(slope or 0.0),
+                                 gy.numel() // c, c, out.data_ptr(), gb.data_ptr(), ws.data_ptr(), nbytes, _stream(gy)))
+        return out, gb if want_bias else None
+    if slope is not None:
+        gy = (gy.float() * torch.where(y > 0, 1.0, slope)).to(torch.bfloat16).contiguous()
+    else:
+        gy = gy.to(torch.bfloat16).contiguous()
+    return gy, gy.float().sum(dim=(0, 1, 2, 3)) if want_bias else None
 
 
 class Conv3(torch.autograd.Function):
@@ -176,9 +240,7 @@ class Conv3(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x0, x1, weight, bias, slope):
         dims = tuple(x0.shape[1:4])
-        cout = weight.shape[0]
-        wmat = weight.permute(0, 2, 3, 4, 1).reshape(cout, -1)
-        y = igemm(x0, x1, 3, 1, 1, dims, wmat, bias, act=slope is not None, slope=slope or 0.0)
+        y = igemm(x0, x1, 3, 1, 1, dims, _pack(weight, (0, 2, 3, 4, 1), 1), bias, act=slope is not None, slope=slope or 0.0)
         ctx.save_for_backward(x0, x1, weight, y)
         ctx.slope = slope
         return y
@@ -186,23 +248,20 @@ class Conv3(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x0, x1, weight, y = ctx.saved_tensors
-        gy = _lrelu_grad(gy, y, ctx.slope) if ctx.slope is not None else gy.to(torch.bfloat16).contiguous()
+        gy, gb = _act_grad(gy, y, ctx.slope, ctx.needs_input_grad[3])
         dims = tuple(x0.shape[1:4])
         cout, cin = weight.shape[:2]
-        gx0 = gx1 = gw = gb = None
+        gx0 = gx1 = gw = None
         if ctx.needs_input_grad[0] or ctx.needs_input_grad[1]:
             # dX[i] = sum_d dY[i + d - 1] W[:, :, 2 - d]: a periodic convolution of dY
             # with the flipped, transposed kernel.
-            wt = weight.flip(2, 3, 4).transpose(0, 1)              # (Cin, Cout, 3, 3, 3)
-            gx = igemm(gy, None, 3, 1, 1, dims, wt.permute(0, 2, 3, 4, 1).reshape(cin, -1))
+            gx = igemm(gy, None, 3, 1, 1, dims, _pack(weight, (1, 2, 3, 4, 0), 1, flip=True))
             c0 = x0.shape[-1]
             gx0 = gx[..., :c0].contiguous() if x1 is not None else gx
             gx1 = gx[..., c0:].contiguous() if x1 is not None else None
         if ctx.needs_input_grad[2]:
             m = wgrad(x0, x1, 3, 1, 1, dims, gy)                   # (27 * Cin, Cout)
             gw = m.reshape(3, 3, 3, cin, cout).permute(4, 3, 0, 1, 2).contiguous()
-        if ctx.needs_input_grad[3]:
-            gb = gy.float().sum(dim=(0, 1, 2, 3))
         return gx0, gx1, gw, gb, None
 
 
@@ -212,8 +271,7 @@ class Down2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, slope):
         dims = tuple(d // 2 for d in x.shape[1:4])
-        cout = weight.shape[0]
-        y = igemm(x, None, 2, 2, 0, dims, weight.permute(0, 2, 3, 4, 1).reshape(cout, -1), bias,
+        y = igemm(x, None, 2, 2, 0, dims, _pack(weight, (0, 2, 3, 4, 1), 1), bias,
                   act=slope is not None, slope=slope or 0.0)
         ctx.save_for_backward(x, weight, y)
         ctx.slope = slope
@@ -222,19 +280,16 @@ class Down2(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, weight, y = ctx.saved_tensors
-        gy = _lrelu_grad(gy, y, ctx.slope) if ctx.slope is not None else gy.to(torch.bfloat16).contiguous()
+        gy, gb = _act_grad(gy, y, ctx.slope, ctx.needs_input_grad[2])
         cdims = tuple(gy.shape[1:4])
         cout, cin = weight.shape[:2]
-        gx = gw = gb = None
+        gx = gw = None
         if ctx.needs_input_grad[0]:
             # dX[2c + d][ci] = sum_co dY[c][co] W[co, ci, d]: scatter into the 8 fine voxels.
-            wm = weight.permute(2, 3, 4, 1, 0).reshape(8 * cin, cout)
-            gx = igemm(gy, None, 1, 1, 0, cdims, wm, mode=OUT_SCATTER2)
+            gx = igemm(gy, None, 1, 1, 0, cdims, _pack(weight, (2, 3, 4, 1, 0), 4), mode=OUT_SCATTER2)
         if ctx.needs_input_grad[1]:
             m = wgrad(x, None, 2, 2, 0, cdims, gy)                 # (8 * Cin, Cout)
             gw = m.reshape(2, 2, 2, cin, cout).permute(4, 3, 0, 1, 2).contiguous()
-        if ctx.needs_input_grad[2]:
-            gb = gy.float().sum(dim=(0, 1, 2, 3))
         return gx, gw, gb, None
 
 
@@ -245,9 +300,8 @@ class Up2(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, slope):
         cdims = tuple(x.shape[1:4])
-        cin, cout = weight.shape[:2]
-        wm = weight.permute(2, 3, 4, 1, 0).reshape(8 * cout, cin)   # n = tap * Cout + co
-        y = igemm(x, None, 1, 1, 0, cdims, wm, bias, mode=OUT_SCATTER2, act=slope is not None,
+        # n = tap * Cout + co
+        y = igemm(x, None, 1, 1, 0, cdims, _pack(weight, (2, 3, 4, 1, 0), 4), bias, mode=OUT_SCATTER2, act=slope is not None,
                   slope=slope or 0.0)
         ctx.save_for_backward(x, weight, y)
         ctx.slope = slope
@@ -256,19 +310,16 @@ class Up2(torch.autograd.Function):
     @staticmethod
     def backward(ctx, gy):
         x, weight, y = ctx.saved_tensors
-        gy = _lrelu_grad(gy, y, ctx.slope) if ctx.slope is not None else gy.to(torch.bfloat16).contiguous()
+        gy, gb = _act_grad(gy, y, ctx.slope, ctx.needs_input_grad[2])
         cdims = tuple(x.shape[1:4])
         cin, cout = weight.shape[:2]
-        gx = gw = gb = None
+        gx = gw = None
         if ctx.needs_input_grad[0]:
             # dX[c][ci] = sum_{d, co} dY[2c + d][co] W[ci, co, d]: a stride-2 gather of dY.
-            wm = weight.permute(0, 2, 3, 4, 1).reshape(cin, 8 * cout)
-            gx = igemm(gy, None, 2, 2, 0, cdims, wm)
+            gx = igemm(gy, None, 2, 2, 0, cdims, _pack(weight, (0, 2, 3, 4, 1), 1))
         if ctx.needs_input_grad[1]:
             m = wgrad(gy, None, 2, 2, 0, cdims, x)                 # (8 * Cout, Cin)
             gw = m.reshape(2, 2, 2, cout, cin).permute(4, 3, 0, 1, 2).contiguous()
-        if ctx.needs_input_grad[2]:
-            gb = gy.float().sum(dim=(0, 1, 2, 3))
         return gx, gw, gb, None
 
 
@@ -287,8 +338,7 @@ def up2(x, weight, bias, slope=None):
 def conv3_f32(x, weight, bias):
     """3x3x3 periodic convolution with an fp32 output (the operator's head)."""
     dims = tuple(x.shape[1:4])
-    cout = weight.shape[0]
-    return igemm(x, None, 3, 1, 1, dims, weight.permute(0, 2, 3, 4, 1).reshape(cout, -1), bias, mode=OUT_F32)
+    return igemm(x, None, 3, 1, 1, dims, _pack(weight, (0, 2, 3, 4, 1), 1), bias, mode=OUT_F32)
 
 
 def info():
