@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <cstdint>
 #include <string>
+#include <utility>
 #include "kernels.cuh"
 #include "color.cuh"
 #include "resident.cuh"
@@ -72,11 +73,13 @@ void set_global_error(const std::string& msg);
 // the previous kernel of the stream has completed and calls pdl_wait() before
 // it touches anything an earlier kernel writes or reads.
 template <class... P, class... A>
-void launch_pdl(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t s, A&&... args)
+void launch_pdl_shared(void (*kernel)(P...), unsigned blocks, unsigned threads, size_t shared, cudaStream_t s,
+                       A&&... args)
 {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = shared;
     cfg.stream = s;
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -84,6 +87,12 @@ void launch_pdl(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStr
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+void launch_pdl(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t s, A&&... args)
+{
+    launch_pdl_shared(kernel, blocks, threads, 0, s, std::forward<A>(args)...);
 }
 
 inline unsigned blocks_for(uint32_t n, unsigned threads) { return (n + threads - 1) / threads; }
