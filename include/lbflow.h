@@ -269,7 +269,7 @@ void *lbf_stream(const lbf_engine *e);
 
 /* ---- Batched geometries ----------------------------------------------------
  * Many independent single-phase D3Q19 geometries of uneven size advanced
- * together: one launch per step walks a packed list of fluid-node tiles of all
+ * together: one launch per step over a packed list of fluid-node tiles of all
  * active geometries (all-solid regions produce no tiles), each tile using its
  * geometry's size and relaxation time; plain steps are replayed from a CUDA
  * graph; per-geometry reductions let each geometry converge and retire on its
@@ -298,9 +298,9 @@ int lbf_batch_convergence(lbf_batch *b, int first, double *out);
 int lbf_batch_flux_sums(lbf_batch *b, double *out);
 /* active[count]: 0 retires a geometry from the step schedule. */
 int lbf_batch_set_active(lbf_batch *b, const uint8_t *active);
-/* Times tile size and grid shape candidates over `steps` steps each and keeps
- * the fastest; the populations are restored afterwards.  out = { threads,
- * tile nodes, 128-thread blocks per SM, ms per step }. */
+/* Times the block sizes (128 and 256 threads, one node each) over `steps`
+ * steps each and keeps the faster; the populations are restored afterwards.
+ * out = { threads, tile nodes, 128-thread blocks per SM, ms per step }. */
 int lbf_batch_autotune(lbf_batch *b, uint32_t steps, double out[4]);
 /* Dense fields of one geometry from the last step that wrote macros. */
 int lbf_batch_get_macros(lbf_batch *b, uint32_t geometry, double *rho, double *u);

@@ -5,9 +5,9 @@
 // geometry keeps its own occupancy words, whose prefix counts start at
 // node_base_g, so the single-geometry pull lookup returns global node
 // indices unchanged.  The node list is cut into tiles of consecutive nodes of
-// one geometry (all-solid regions produce no nodes and so no tiles); a grid of
-// resident blocks walks the tile list of the still-active geometries every
-// step, reading each tile's geometry size and collision rates.  Steps are
+// one geometry (all-solid regions produce no nodes and so no tiles); a step is
+// one block per tile of the still-active geometries, reading the tile's
+// geometry size and collision rates.  Steps are
 // replayed from a captured CUDA graph.  FP16 storage rounds stochastically
 // with the single engine's per-step seeds: the step count lives in device
 // memory (a pair of words indexed by the buffer parity: a step reads one and
@@ -15,8 +15,8 @@
 // see a new seed every step without any host involvement.  Per-geometry reductions write one
 // partial per tile and then sum each geometry's tiles in order
 // (deterministic), so every geometry can be tested for convergence and
-// retired on its own.  lbf_batch_autotune picks the tile size and grid shape
-// by timing candidates on the batch itself.
+// retired on its own.  lbf_batch_autotune picks the tile size by timing the
+// candidates on the batch itself.
 #include "../../include/lbflow.h"
 #include "internal.h"
 #include "reduce.cuh"
@@ -45,43 +45,53 @@ thread_local std::string g_batch_error;
 
 int bfail(lbf_batch* b, int code, const std::string& m);
 
-template <class L, class S, bool PULL>
-__global__ void __launch_bounds__(256)
-batch_step(const BatchGeom* __restrict__ geoms, const Tile* __restrict__ tiles, uint32_t ntiles,
-           const uint2* __restrict__ occ, const uint32_t* __restrict__ coord, uint32_t nfp,
-           const Force F, const double rho0, const typename S::T* __restrict__ fin,
-           typename S::T* __restrict__ fout, Macros mo, const int out, uint32_t* __restrict__ err,
-           uint32_t* __restrict__ step_count, const int parity)
+// Resident blocks of TH threads per SM the kernel is compiled for: the single
+// geometry's step (StepBlocks), at 256 threads rounded down.
+template <class S, int TH> struct BatchBlocks { static constexpr int value = StepBlocks<S>::value * 128 / TH; };
+
+// One tile of at most TH nodes per block: the step kernel of a single geometry
+// with the tile's geometry looked up.  Its register cap, block count and
+// programmatic dependent launch hide the gather's latency better than resident
+// blocks at the compiler's register count that walk the tile list (48 media of
+// edges 32-96, 2.1 M nodes, us per step: FP64 136 -> 120, FP32 98 -> 70, FP16
+// 89 -> 69; 48 of edges 32-48, 0.67 M nodes, FP64 44.6 -> 40.5).  FP64 looks
+// its sources up as the single step does (all branch-free: 126).  Only the
+// values that earlier launches write are behind the wait.
+template <class L, class S, bool PULL, int TH>
+__global__ void __launch_bounds__(TH, BatchBlocks<S, TH>::value)
+batch_step(const BatchGeom* __restrict__ geoms, const Tile* __restrict__ tiles, const uint2* __restrict__ occ,
+           const uint32_t* __restrict__ coord, uint32_t nfp, const Force F, const double rho0,
+           const double inv_rho0, const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+           Macros mo, const int out, uint32_t* __restrict__ err, uint32_t* __restrict__ step_count,
+           const int parity)
 {
+    pdl_trigger();
+    const Tile tl = tiles[blockIdx.x];
+    const BatchGeom& G = geoms[tl.geom];
+    Grid g;
+    g.nx = G.nx; g.ny = G.ny; g.nz = G.nz; g.W = G.W;
+    g.nf = 0;
+    g.nfp = nfp;
+    g.occ = occ + G.occ_base;
+    g.coord = coord;
+    ScspParams P;
+    P.rho0 = rho0;
+    P.inv_rho0 = inv_rho0;
+    P.rate.sp = G.sp;
+    P.rate.sm = G.sm;
+    P.node0 = G.node_base;
     // Stochastic rounding seed of this step (16-bit float storage, pull
     // steps): count k = 1, 2, ... of pull steps, as the single engine seeds
     // them.  This launch reads step_count[parity] and publishes k into
     // step_count[parity ^ 1] for the next launch, never the word it reads.
-    uint32_t seed = 0;
     if (S::dither && PULL && step_count) {
+        pdl_wait();
         const uint32_t k = step_count[parity] + 1u;
-        seed = (k * 2654435761u) | 1u;
+        P.seed = (k * 2654435761u) | 1u;
         if (blockIdx.x == 0 && threadIdx.x == 0) step_count[parity ^ 1] = k;
     }
-    for (uint32_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const Tile tl = tiles[t];
-        const BatchGeom G = geoms[tl.geom];
-        Grid g;
-        g.nx = G.nx; g.ny = G.ny; g.nz = G.nz; g.W = G.W;
-        g.nf = G.node_base + G.nf;
-        g.nfp = nfp;
-        g.occ = occ + G.occ_base;
-        g.coord = coord;
-        ScspParams P;
-        P.rho0 = rho0;
-        P.inv_rho0 = 1.0 / rho0;
-        P.rate.sp = G.sp;
-        P.rate.sm = G.sm;
-        P.seed = seed;
-        P.node0 = G.node_base;
-        for (uint32_t k = threadIdx.x; k < tl.count; k += blockDim.x)
-            scsp_update<L, S, PULL, true>(g, F, P, fin, fout, tl.first + k, mo, out, err, nullptr, nullptr);
-    }
+    if (threadIdx.x < tl.count)
+        scsp_update<L, S, PULL>(g, F, P, fin, fout, tl.first + threadIdx.x, mo, out, err, nullptr, nullptr);
 }
 
 // Per-tile partial sums of a reduction functor (one block per tile).
@@ -116,21 +126,35 @@ tile_sums(const Fn fn, const Tile* __restrict__ tiles, double* __restrict__ part
     }
 }
 
-// Sum each geometry's tile partials in tile order (one thread per geometry).
+// Sum of each geometry's tile partials, one warp per geometry: every lane adds
+// every 32nd tile in order, then a fixed tree (deterministic).  One thread per
+// geometry walked its tiles alone, K dependent loads each: 2.5 ms for 48 media
+// of edges 32-96, 1 % of it memory time.
 template <class Fn>
-__global__ void geom_sums(const double* __restrict__ partial, const uint32_t* __restrict__ tile_first,
-                          const uint32_t* __restrict__ tile_count, uint32_t ngeom, double* __restrict__ out)
+__global__ void __launch_bounds__(32)
+geom_sums(const double* __restrict__ partial, const uint32_t* __restrict__ tile_first,
+          const uint32_t* __restrict__ tile_count, double* __restrict__ out)
 {
     constexpr int K = Fn::K;
-    const uint32_t gi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (gi >= ngeom) return;
-    for (int k = 0; k < K; ++k) {
-        double v = 0.0;
-        for (uint32_t t = 0; t < tile_count[gi]; ++t) {
-            const double p = partial[(size_t)(tile_first[gi] + t) * K + k];
-            v = Fn::is_max(k) ? fmax(v, p) : v + p;
+    const uint32_t first = tile_first[blockIdx.x], count = tile_count[blockIdx.x];
+    double v[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = 0.0;
+    for (uint32_t t = threadIdx.x; t < count; t += 32) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const double p = partial[(size_t)(first + t) * K + k];
+            v[k] = Fn::is_max(k) ? fmax(v[k], p) : v[k] + p;
         }
-        out[(size_t)gi * K + k] = v;
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double p = __shfl_down_sync(0xffffffffu, v[k], o);
+            v[k] = Fn::is_max(k) ? fmax(v[k], p) : v[k] + p;
+        }
+        if (threadIdx.x == 0) out[(size_t)blockIdx.x * K + k] = v[k];
     }
 }
 
@@ -169,8 +193,7 @@ struct lbf_batch {
     std::vector<uint32_t> tile_first, tile_count;
     Force force{};
     cudaStream_t stream = nullptr;
-    // launch shape (autotuned)
-    unsigned threads = 128, tile_nodes = 256, grid = 0;
+    unsigned threads = 128;   // threads per block = nodes per tile: 128 or 256 (autotuned)
     // CUDA graph of `graph_steps` plain steps
     cudaGraphExec_t graph = nullptr;
     uint32_t graph_steps = 0;
@@ -202,31 +225,35 @@ Macros batch_macros(const lbf_batch* b)
 }
 
 template <class S>
-void launch_batch(lbf_batch* b, bool pull, int out, const Tile* tiles, uint32_t ntiles, unsigned grid)
+void launch_batch(lbf_batch* b, bool pull, int out, const Tile* tiles, uint32_t ntiles)
 {
     using T = typename S::T;
     if (!ntiles) return;
-    const T* fin = (const T*)b->f[b->cur];
-    T* fout = (T*)b->f[b->cur ^ 1];
-    if (pull)
-        batch_step<D3Q19, S, true><<<grid, b->threads, 0, b->stream>>>(
-            b->d_geoms, tiles, ntiles, b->d_occ, b->d_coord, b->nfp, b->force, b->rho0, fin, fout,
-            batch_macros(b), out, b->err, b->d_step, b->cur);
-    else
-        batch_step<D3Q19, S, false><<<grid, b->threads, 0, b->stream>>>(
-            b->d_geoms, tiles, ntiles, b->d_occ, b->d_coord, b->nfp, b->force, b->rho0, fin, fout,
-            batch_macros(b), out, b->err, b->d_step, b->cur);
+    auto step = [&](auto kernel) {
+        launch_pdl(kernel, ntiles, b->threads, b->stream, b->d_geoms, tiles, b->d_occ, b->d_coord, b->nfp, b->force,
+                   b->rho0, 1.0 / b->rho0, (const T*)b->f[b->cur], (T*)b->f[b->cur ^ 1], batch_macros(b), out, b->err,
+                   b->d_step, b->cur);
+    };
+    if (b->threads == 128) step(pull ? batch_step<D3Q19, S, true, 128> : batch_step<D3Q19, S, false, 128>);
+    else step(pull ? batch_step<D3Q19, S, true, 256> : batch_step<D3Q19, S, false, 256>);
+}
+
+// Resident 128-thread blocks' worth per SM of the current shape.
+double batch_blocks(const lbf_batch* b)
+{
+    const bool f64 = b->storage == LBF_STORE_FP64;
+    if (b->threads == 128) return f64 ? BatchBlocks<StoreF64, 128>::value : BatchBlocks<StoreF32<D3Q19>, 128>::value;
+    return 2.0 * (f64 ? BatchBlocks<StoreF64, 256>::value : BatchBlocks<StoreF32<D3Q19>, 256>::value);
 }
 
 void batch_launch(lbf_batch* b, bool pull, int out, bool all_tiles = false)
 {
     const Tile* tiles = all_tiles ? b->d_tiles_all : b->d_tiles_active;
     const uint32_t n = all_tiles ? b->ntiles_all : b->ntiles_active;
-    const unsigned grid = std::max(1u, std::min(b->grid, n));
     switch (b->storage) {
-    case LBF_STORE_FP64: launch_batch<StoreF64>(b, pull, out, tiles, n, grid); break;
-    case LBF_STORE_FP16: launch_batch<StoreF16<D3Q19>>(b, pull, out, tiles, n, grid); break;
-    default: launch_batch<StoreF32<D3Q19>>(b, pull, out, tiles, n, grid); break;
+    case LBF_STORE_FP64: launch_batch<StoreF64>(b, pull, out, tiles, n); break;
+    case LBF_STORE_FP16: launch_batch<StoreF16<D3Q19>>(b, pull, out, tiles, n); break;
+    default: launch_batch<StoreF32<D3Q19>>(b, pull, out, tiles, n); break;
     }
     b->cur ^= 1;
 }
@@ -247,8 +274,8 @@ int build_tiles(lbf_batch* b)
     for (uint32_t g = 0; g < b->count; ++g) {
         b->tile_first[g] = (uint32_t)b->tiles_all.size();
         const BatchGeom& G = b->geoms[g];
-        for (uint32_t k = 0; k < G.nf; k += b->tile_nodes)
-            b->tiles_all.push_back(Tile{g, G.node_base + k, std::min(b->tile_nodes, G.nf - k)});
+        for (uint32_t k = 0; k < G.nf; k += b->threads)
+            b->tiles_all.push_back(Tile{g, G.node_base + k, std::min(b->threads, G.nf - k)});
         b->tile_count[g] = (uint32_t)b->tiles_all.size() - b->tile_first[g];
     }
     b->ntiles_all = (uint32_t)b->tiles_all.size();
@@ -317,9 +344,8 @@ template <class Fn>
 int batch_reduce(lbf_batch* b, const Fn& fn, double* out)
 {
     if (!b->ntiles_all) { std::memset(out, 0, sizeof(double) * Fn::K * b->count); return LBF_OK; }
-    tile_sums<Fn><<<b->ntiles_all, 256, 0, b->stream>>>(fn, b->d_tiles_all, b->d_partial);
-    geom_sums<Fn><<<(b->count + 127) / 128, 128, 0, b->stream>>>(b->d_partial, b->d_tile_first, b->d_tile_count,
-                                                                 b->count, b->d_out);
+    tile_sums<Fn><<<b->ntiles_all, 128, 0, b->stream>>>(fn, b->d_tiles_all, b->d_partial);
+    geom_sums<Fn><<<b->count, 32, 0, b->stream>>>(b->d_partial, b->d_tile_first, b->d_tile_count, b->d_out);
     BCK(b, cudaGetLastError());
     BCK(b, cudaMemcpyAsync(out, b->d_out, sizeof(double) * Fn::K * b->count, cudaMemcpyDeviceToHost, b->stream));
     BCK(b, cudaStreamSynchronize(b->stream));
@@ -466,9 +492,6 @@ int lbf_batch_create(const lbf_batch_geometry* geoms, uint32_t count, const lbf_
     b->force.fx = F0[0]; b->force.fy = F0[1]; b->force.fz = F0[2];
     b->force.label = b->d_label;
     b->force.label_force = b->d_label_force;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    b->grid = (unsigned)sms * 8;
     if (int rc = build_tiles(b)) { std::string m = b->last_error; lbf_batch_destroy(b); return bfail(nullptr, rc, m); }
     *out = b;
     return LBF_OK;
@@ -569,15 +592,10 @@ int lbf_batch_autotune(lbf_batch* b, uint32_t steps, double out[4])
     if (!b || !out) return bfail(b, LBF_EINVAL, "NULL argument");
     if (!b->initialized) return bfail(b, LBF_ESTATE, "autotune before lbf_batch_initialize");
     BCK(b, cudaSetDevice(b->device));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
     if (steps < 2) steps = 2;
     steps += steps & 1;   // even: the populations end in the buffer they started in
-    const unsigned threads_c[] = {128, 256};
-    const unsigned tile_mult[] = {1, 2, 4};
-    const unsigned per_sm[] = {4, 8, 16};
     double best = 1e300;
-    unsigned bt = b->threads, btile = b->tile_nodes, bgrid = b->grid;
+    unsigned bt = b->threads;
     // Trials advance the populations; keep a copy and put it back afterwards
     // so that tuning leaves the simulation where it was.
     const size_t fbytes = (size_t)19 * b->nfp * b->elem;
@@ -589,23 +607,19 @@ int lbf_batch_autotune(lbf_batch* b, uint32_t steps, double out[4])
     cudaEvent_t e0, e1;
     BCK(b, cudaEventCreate(&e0));
     BCK(b, cudaEventCreate(&e1));
-    for (unsigned th : threads_c)
-        for (unsigned tm : tile_mult)
-            for (unsigned ps : per_sm) {
-                b->threads = th;
-                b->tile_nodes = th * tm;
-                b->grid = (unsigned)sms * ps * 128 / th;
-                if (int rc = build_tiles(b)) return rc;
-                batch_launch(b, true, 0);          // warm
-                batch_launch(b, true, 0);
-                cudaEventRecord(e0, b->stream);
-                for (uint32_t s = 0; s < steps; ++s) batch_launch(b, true, 0);
-                cudaEventRecord(e1, b->stream);
-                BCK(b, cudaEventSynchronize(e1));
-                float ms = 0;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (ms < best) { best = ms; bt = th; btile = th * tm; bgrid = b->grid; }
-            }
+    for (unsigned th : {128u, 256u}) {
+        b->threads = th;
+        if (int rc = build_tiles(b)) return rc;
+        batch_launch(b, true, 0);          // warm
+        batch_launch(b, true, 0);
+        cudaEventRecord(e0, b->stream);
+        for (uint32_t s = 0; s < steps; ++s) batch_launch(b, true, 0);
+        cudaEventRecord(e1, b->stream);
+        BCK(b, cudaEventSynchronize(e1));
+        float ms = 0;
+        cudaEventElapsedTime(&ms, e0, e1);
+        if (ms < best) { best = ms; bt = th; }
+    }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     BCK(b, cudaMemcpyAsync(b->f[b->cur], snap, fbytes, cudaMemcpyDeviceToDevice, b->stream));
@@ -614,10 +628,8 @@ int lbf_batch_autotune(lbf_batch* b, uint32_t steps, double out[4])
     cudaFree(snap);
     if (b->cur != cur0) return bfail(b, LBF_ESTATE, "autotune: buffer parity changed");
     b->threads = bt;
-    b->tile_nodes = btile;
-    b->grid = bgrid;
     if (int rc = build_tiles(b)) return rc;
-    out[0] = bt; out[1] = btile; out[2] = (double)bgrid / sms; out[3] = best / steps;
+    out[0] = bt; out[1] = bt; out[2] = batch_blocks(b); out[3] = best / steps;
     BCK(b, cudaGetLastError());
     return LBF_OK;
 }
