@@ -16,6 +16,7 @@ Three operators:
   up2    2x2x2 transposed convolution with stride 2 (doubles the grid)
 """
 import ctypes
+import functools
 import math
 
 import torch
@@ -72,7 +73,7 @@ def _lib():
 
 def error_word(device):
     """The device error word the kernels of this device report into."""
-    key = torch.device(device).index or 0
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
     if key not in _ERR:
         _ERR[key] = torch.zeros(1, dtype=torch.int32, device=device)
     return _ERR[key]
@@ -87,7 +88,7 @@ def check(device=None):
 
 
 def _stream(t):
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(t.device.index)
 
 
 def _ck(rc):
@@ -142,19 +143,26 @@ def _pack(weight, order, split, flip=False):
         n = math.prod(w.shape[:split])
         mat = w.reshape(n, -1)
         return _Packed(pack_weight(mat), *mat.shape)
-    dims = [weight.shape[d] for d in order]
-    strides = [weight.stride(d) for d in order]
-    at = weight.data_ptr()
+    dims, strides, n, k, n_pad, k_pad, offset = _pack_plan(weight.shape, weight.stride(), order, split, flip)
+    out = torch.empty(n_pad, k_pad, dtype=torch.bfloat16, device=weight.device)
+    _ck(_lib().lbf_pack_weight(weight.data_ptr() + offset, dims, strides, split, out.data_ptr(), n_pad, k_pad,
+                               _stream(weight)))
+    return _Packed(out, n, k)
+
+
+@functools.lru_cache(maxsize=256)
+def _pack_plan(shape, stride, order, split, flip):
+    """Extents, strides and matrix sizes of _pack for a weight of this shape."""
+    dims = [shape[d] for d in order]
+    strides = [stride[d] for d in order]
+    offset = 0
     if flip:
         for j, d in enumerate(order):
             if d >= 2:
-                at += 4 * strides[j] * (dims[j] - 1)
+                offset += 4 * strides[j] * (dims[j] - 1)
                 strides[j] = -strides[j]
     n, k = math.prod(dims[:split]), math.prod(dims[split:])
-    out = torch.empty(_pad16(n), _pad64(k), dtype=torch.bfloat16, device=weight.device)
-    _ck(_lib().lbf_pack_weight(at, (U32 * 5)(*dims), (ctypes.c_int64 * 5)(*strides), split, out.data_ptr(),
-                               out.shape[0], out.shape[1], _stream(weight)))
-    return _Packed(out, n, k)
+    return (U32 * 5)(*dims), (ctypes.c_int64 * 5)(*strides), n, k, _pad16(n), _pad64(k), offset
 
 
 def igemm(src0, src1, ksize, stride, pad, out_dims, wmat, bias=None, mode=OUT_BF16, out=None, out_ld=None,
