@@ -1326,6 +1326,8 @@ bool resident_ok(lbf_engine* e)
     return cudaStreamIsCapturing(e->stream, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
+constexpr uint32_t kResidentSteps = 1024;
+
 // Queues the steps; false, with nothing queued, where the device cannot take
 // the launch or the words' memory: the caller then launches step by step.
 bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
@@ -1369,8 +1371,18 @@ int lbf_step(lbf_engine* e, uint32_t nsteps, uint32_t flags)
     int rc = setdev(e);
     if (rc) return rc;
     const int out = (flags & LBF_STEP_MACROS ? kOutMacros : 0) | (flags & LBF_STEP_ADJACENT ? kOutAdjacent : 0);
-    if (nsteps > 1 && resident_ok(e) && resident_steps(e, nsteps, out)) return LBF_OK;
-    for (uint32_t s = 0; s < nsteps; ++s) launch_step(e, true, s + 1 == nsteps ? out : 0);
+    uint32_t s = 0;
+    if (nsteps > 1 && resident_ok(e)) {
+        // A launch holds its part of the GPU to its end: at most kResidentSteps
+        // steps (a few milliseconds) each, so that other streams get their turn.
+        while (s < nsteps) {
+            uint32_t m = std::min(nsteps - s, kResidentSteps);
+            if (nsteps - s - m == 1) --m;      // a launch takes at least two steps
+            if (!resident_steps(e, m, s + m == nsteps ? out : 0)) break;
+            s += m;
+        }
+    }
+    for (; s < nsteps; ++s) launch_step(e, true, s + 1 == nsteps ? out : 0);
     LBF_CK(e, cudaGetLastError());
     return LBF_OK;
 }

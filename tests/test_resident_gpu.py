@@ -57,3 +57,14 @@ def test_largest_geometries(storage, shape):
     many = _state(g, storage, 'MRT', [9])
     for a, b in zip(one, many):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize('storage', ['fp64', 'fp16'])
+@pytest.mark.parametrize('steps', [1023, 1024, 1025, 2049])
+def test_calls_of_several_launches(storage, steps):
+    """A resident launch takes at most 1,024 steps and at least two."""
+    g = _geometry((3, 5, 7), 0.9, two_forces=False)
+    one = _state(g, storage, 'MRT', [1] * steps)
+    many = _state(g, storage, 'MRT', [steps])
+    for a, b in zip(one[:3], many[:3]):
+        assert np.array_equal(a, b)
