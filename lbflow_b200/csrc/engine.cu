@@ -51,8 +51,8 @@ struct lbf_engine {
     double* solid_f[2] = {nullptr, nullptr};   // populations of solid voxels (lbf_keep_solid_populations)
     int scur = 0;
     size_t ns = 0;                  // solid voxels (N - nf)
-    double* red = nullptr;
-    double* h_red = nullptr;        // pinned
+    uint32_t* red_done = nullptr;   // blocks finished in a running reduction
+    double* h_red = nullptr;        // page-locked; reductions write their results here
     cudaStream_t stream = nullptr;
     Force force{};
     ZouHe zh{};                     // PB/VB boundary nodes (single phase)
@@ -271,16 +271,28 @@ void launch_step(lbf_engine* e, bool pull, int out)
     e->cur ^= 1;
 }
 
+// Queues a reduction into h_red; queued device work that follows runs before
+// finish_reduce returns, too.
+template <class Fn>
+int start_reduce(lbf_engine* e, const Fn& fn)
+{
+    reduce_nodes<Fn><<<kReduceBlocks, kReduceThreads, 0, e->stream>>>(fn, e->nf, e->partial, e->red_done, e->h_red);
+    LBF_CK(e, cudaGetLastError());
+    return LBF_OK;
+}
+
+int finish_reduce(lbf_engine* e, double* out, int k)
+{
+    LBF_CK(e, cudaStreamSynchronize(e->stream));
+    std::memcpy(out, e->h_red, k * sizeof(double));
+    return LBF_OK;
+}
+
 template <class Fn>
 int run_reduce(lbf_engine* e, const Fn& fn, double* out)
 {
-    reduce_pass1<Fn><<<kReduceBlocks, kReduceThreads, 0, e->stream>>>(fn, e->nf, e->partial);
-    reduce_pass2<Fn><<<1, kReduceThreads, 0, e->stream>>>(e->partial, kReduceBlocks, e->red);
-    LBF_CK(e, cudaGetLastError());
-    LBF_CK(e, cudaMemcpyAsync(e->h_red, e->red, Fn::K * sizeof(double), cudaMemcpyDeviceToHost, e->stream));
-    LBF_CK(e, cudaStreamSynchronize(e->stream));
-    std::memcpy(out, e->h_red, Fn::K * sizeof(double));
-    return LBF_OK;
+    const int rc = start_reduce(e, fn);
+    return rc ? rc : finish_reduce(e, out, Fn::K);
 }
 
 // Stored populations <-> dense-per-node FP64 ([phase][q][nfp]).
@@ -1021,7 +1033,8 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
     LBF_ALLOC(e->err, 1);
     LBF_CUDA(cudaMemsetAsync(e->err, 0, sizeof(uint32_t), e->stream));
     LBF_ALLOC(e->partial, (size_t)kReduceBlocks * kReduceMaxK);
-    LBF_ALLOC(e->red, kReduceMaxK);
+    LBF_ALLOC(e->red_done, 1);
+    LBF_CUDA(cudaMemsetAsync(e->red_done, 0, sizeof(uint32_t), e->stream));
 
     e->force.uniform = uniform ? 1 : 0;
     e->force.fx = F0[0]; e->force.fy = F0[1]; e->force.fz = F0[2];
@@ -1139,7 +1152,7 @@ void lbf_destroy(lbf_engine* e)
     if (e->stream) cudaStreamSynchronize(e->stream);
     void* ptrs[] = {e->f[0], e->f[1], e->ex[0], e->ex[1], e->occ, e->coord, e->node_label, e->node_phase, e->label_force,
                     e->rho0, e->rho1, e->u, e->uprev, e->uadj, e->ind, e->indprev, e->indadj,
-                    e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red,
+                    e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red_done,
                     e->zh_node, e->zh_code, e->zh_bits, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
                     e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words,
                     e->link_row, e->link_mask, e->link_base};
@@ -1604,15 +1617,12 @@ int lbf_convergence(lbf_engine* e, int first, double out[6])
     const bool color = e->cfg.model == LBF_MODEL_COLOR;
     if (!first) {
         ConvergenceFn fn{e->u, e->uprev, e->uadj, e->ind, e->indprev, e->indadj, e->nfp, color ? 1 : 0};
-        double r[ConvergenceFn::K];
-        if ((rc = run_reduce(e, fn, r))) return rc;
-        for (int k = 0; k < ConvergenceFn::K; ++k) out[k] = r[k];
+        if ((rc = start_reduce(e, fn))) return rc;
     }
     LBF_CK(e, cudaMemcpyAsync(e->uprev, e->u, 3 * (size_t)e->nfp * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
     if (color)
         LBF_CK(e, cudaMemcpyAsync(e->indprev, e->ind, (size_t)e->nfp * sizeof(double), cudaMemcpyDeviceToDevice, e->stream));
-    LBF_CK(e, cudaStreamSynchronize(e->stream));
-    return LBF_OK;
+    return finish_reduce(e, out, first ? 0 : ConvergenceFn::K);
 }
 
 int lbf_report_sums(lbf_engine* e, uint32_t axis, uint32_t lo, uint32_t hi, double out[10])
@@ -1657,8 +1667,9 @@ int lbf_status(lbf_engine* e, uint32_t* bits)
     if (!e || !bits) return fail(e, LBF_EINVAL, "NULL argument");
     int rc = setdev(e);
     if (rc) return rc;
+    LBF_CK(e, cudaMemcpyAsync(e->h_red, e->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
     LBF_CK(e, cudaStreamSynchronize(e->stream));
-    LBF_CK(e, cudaMemcpy(bits, e->err, sizeof(uint32_t), cudaMemcpyDeviceToHost));
+    std::memcpy(bits, e->h_red, sizeof(uint32_t));
     return LBF_OK;
 }
 
