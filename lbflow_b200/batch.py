@@ -237,8 +237,8 @@ def converge_sharded(geometries, taus, labels, g, rank=0, world=1, device=0, col
                      report=1000, tol=1e-6, max_steps=200000, group=None, batch_factory=None):
     """Converge a list of geometries split over `world` processes, one GPU
     each.  Geometries are independent, so there is no data-path collective:
-    every rank runs its share (partition of estimated_work) in its own
-    persistent batched launch, and only the per-geometry results (steps, K,
+    every rank runs its share (partition of estimated_work) as its own
+    batch, and only the per-geometry results (steps, K,
     convergence flag) and each rank's seconds are exchanged afterwards,
     host-side, with torch.distributed.all_gather_object on `group`.
     Returns the results in the original order, seconds = the slowest rank's

@@ -460,12 +460,15 @@ __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constan
 // each is used by the kCZ z slices' accumulators.  The K order per output is
 // igemm's (tap, then channel).
 //
-// Measured, igemm -> here: 16 -> 16 channels at 96^3 238 -> 61 us, 32 -> 16
-// (two sources) 403 -> 104, 32 -> 32 at 48^3 63 -> 22, 64 -> 64 at 2 x 48^3
-// 91 -> 82.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
+// Measured, igemm -> here: 16 -> 16 channels at 96^3 238 -> 48 us, 8 -> 16 187
+// -> 44, 32 -> 16 (two sources) 403 -> 102, 32 -> 32 at 48^3 63 -> 22, 64 -> 64
+// at 2 x 48^3 91 -> 82.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
 // (cp.async at 14 bytes a cycle), 28,000 for 432 MMAs (N = 64, 65 cycles each;
-// operand reads alone need 48), the rest weights and epilogue.  8 producer
-// warps: 16 take 96 us for 16 -> 16, their registers cost a resident block.
+// operand reads alone need 48), the rest weights and epilogue.  Narrow inputs
+// need several resident blocks to overlap those phases: the registers are
+// capped for as many as shared memory holds (16 -> 16 at the compiler's 95
+// registers, two blocks, 60 us; three 51, four 48).  8 producer warps: 16 take
+// 96 us for 16 -> 16, their registers cost a resident block.
 constexpr int kCX = 8, kCY = 16, kCZ = 4;
 constexpr int kHX = kCX + 2, kHY = kCY + 2, kHZ = kCZ + 2;
 constexpr int kHalo = kHX * kHY * kHZ;
@@ -484,7 +487,7 @@ constexpr size_t conv3_smem(uint32_t groups, uint32_t bn, TapRing r) {
 // G: 8-channel groups held (2, 4 or 8; those past the input's channels are
 // zeros).
 template <int BN, int G>
-__global__ void __launch_bounds__(kConvThreads, 1)
+__global__ void __launch_bounds__(kConvThreads, G == 2 ? 4 : (G == 4 ? 2 : 1))
 conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint32_t ty, const uint32_t tz,
              const TapRing ring) {
     extern __shared__ uint8_t smem_raw[];
