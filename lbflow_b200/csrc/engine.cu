@@ -958,6 +958,7 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
             cudaFreeAsync(e->link_base, e->stream);
             e->link_row = e->link_base = nullptr;
             e->link_mask = nullptr;
+            e->bytes -= tiles * (kLinkTile * (sizeof(uint4) + sizeof(uint32_t)) + 2 * sizeof(uint4));
         }
     }
     if (boundaries || c.model == LBF_MODEL_COLOR) {

@@ -42,8 +42,6 @@ struct Resident {
 
 // A population and the number of the step that wrote it, moved as one access.
 struct Word128 { unsigned long long value, tag; };
-template <int BYTES> struct WordOf { using type = unsigned long long; };
-template <> struct WordOf<8> { using type = Word128; };
 
 __device__ __forceinline__ void put_word(Word128* p, double v, uint32_t tag)
 {
