@@ -61,7 +61,7 @@ template <class L, class S, bool PULL, int TH>
 __global__ void __launch_bounds__(TH, BatchBlocks<S, TH>::value)
 batch_step(const BatchGeom* __restrict__ geoms, const Tile* __restrict__ tiles, const uint2* __restrict__ occ,
            const uint32_t* __restrict__ coord, uint32_t nfp, const Force F, const double rho0,
-           const double inv_rho0, const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+           const double inv_rho0, const typename S::T* fin, typename S::T* __restrict__ fout,
            Macros mo, const int out, uint32_t* __restrict__ err, uint32_t* __restrict__ step_count,
            const int parity)
 {

@@ -64,12 +64,12 @@ template <class L, class H> struct ColorPacked {
                                                                  : __float2half_rn(x));
         else return __bfloat16_as_ushort(__float2bfloat16_rz(dither_bits(x, r, 16)));
     }
-    __device__ static void load_pair(const uint16_t* __restrict__ fin, uint32_t off, uint32_t nblk, int q,
+    __device__ static void load_pair(const uint16_t* fin, uint32_t off, uint32_t nblk, int q,
                                      float rho_bar, float& f0, float& f1)
     {
-        const float g = to_f(__ldg(fin + off)) * ShiftScale<L>::inv(q);
+        const float g = to_f(fin[off]) * ShiftScale<L>::inv(q);
         const float fT = (float)L::w36f(q) * (1.0f / 36.0f) * rho_bar + g;
-        const float r = (float)__ldg(fin + nblk + off) * (1.0f / 32768.0f) - 0.5f;
+        const float r = (float)fin[nblk + off] * (1.0f / 32768.0f) - 0.5f;
         f0 = r * fT;
         f1 = fT - f0;
     }
@@ -124,11 +124,11 @@ __device__ __forceinline__ uint32_t film_sources(const Grid& g, const uint32_t* 
 // UINT32_MAX when it is solid (bounce-back).  One neighbour lookup serves both
 // components (the sources are the same).
 template <class L, class S, bool PULL, class Sink>
-__device__ __forceinline__ void color_pull(const Grid& g, const typename S::T* __restrict__ fin, uint32_t i,
+__device__ __forceinline__ void color_pull(const Grid& g, const typename S::T* fin, uint32_t i,
                                            int x, int y, int z, typename S::R rho_bar, Sink&& sink)
 {
     using R = typename S::R;
-    const typename S::T* __restrict__ fin1 = fin + (size_t)L::Q * g.nfp;
+    const typename S::T* fin1 = fin + (size_t)L::Q * g.nfp;
     const uint32_t nfp = g.nfp;
     const uint32_t nblk = (uint32_t)L::Q * nfp;
     auto load2 = [&](uint32_t off, int q, R& a, R& b) {
@@ -171,7 +171,7 @@ __device__ __forceinline__ void color_pull(const Grid& g, const typename S::T* _
 // voxel keeps only its own phase (clearHalfFilm, colorfluid.cpp:752-765).
 // nbr keeps the occupancy neighbours: a film voxel is fluid for the gradient.
 template <class L, class S, bool PULL, bool FILM>
-__device__ __forceinline__ void color_gather(const Grid& g, const Film& film, const typename S::T* __restrict__ fin,
+__device__ __forceinline__ void color_gather(const Grid& g, const Film& film, const typename S::T* fin,
                                              uint32_t i, int x, int y, int z, typename S::R (&f0)[L::Q],
                                              typename S::R (&f1)[L::Q], uint32_t (&nbr)[L::Q],
                                              typename S::R rho_bar = typename S::R(0))
@@ -224,7 +224,7 @@ template <class L> constexpr int normal_codes() { return L::D == 3 ? 11 * 11 * 1
 // Pass 1: phase field.  PULL = false reads the node's own values (t = 0).
 template <class L, class S, bool PULL, bool FILM>
 __global__ void __launch_bounds__(128)
-color_phase(const Grid g, const Film film, const typename S::T* __restrict__ fin, double2* __restrict__ dens,
+color_phase(const Grid g, const Film film, const typename S::T* fin, double2* __restrict__ dens,
             double* __restrict__ phid, uint32_t* __restrict__ err, const double rho_bar)
 {
     using R = typename S::R;
@@ -539,7 +539,7 @@ __device__ __forceinline__ void color_update(const Grid& g, const Force& F, cons
 // each neighbour is one address computation, no occupancy lookup.
 template <class L, class R>
 __device__ __forceinline__ void color_gradient_dense(const Grid& g, const ColorWall& W,
-                                                     const double* __restrict__ phid, const uint32_t i, int x, int y,
+                                                     const double* phid, const uint32_t i, int x, int y,
                                                      int z, R (&gr)[3], R& norm)
 {
     const int xs[3] = {x == 0 ? g.nx - 1 : x - 1, x, x + 1 == g.nx ? 0 : x + 1};
@@ -549,7 +549,7 @@ __device__ __forceinline__ void color_gradient_dense(const Grid& g, const ColorW
 #pragma unroll
     for (int q = 0; q < L::Q; ++q) {
         const size_t v = ((size_t)zs[1 + L::ez(q)] * g.ny + ys[1 + L::ey(q)]) * g.nx + xs[1 + L::ex(q)];
-        phin[q] = R(__ldg(&phid[v]));
+        phin[q] = R(phid[v]);
     }
     color_gradient_node<L, R>(W, i, phin[0], phin, gr, norm);
 }
@@ -570,8 +570,8 @@ template <> struct CollideBlocks<StoreF64> { static constexpr int value = 4; };
 template <class L, class S, int COLL, bool PULL, bool FILM>
 __global__ void __launch_bounds__(128, CollideBlocks<S>::value)
 color_collide(const Grid g, const Film film, const Force F, const ColorParams P, const ColorWall W,
-              const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-              const double2* __restrict__ dens, const double* __restrict__ phid, Macros mo, const int out,
+              const typename S::T* fin, typename S::T* __restrict__ fout,
+              const double2* dens, const double* phid, Macros mo, const int out,
               uint32_t* __restrict__ err)
 {
     using R = typename S::R;
@@ -667,7 +667,7 @@ __device__ __forceinline__ void color_zou_he_node(R (&f0)[L::Q], R (&f1)[L::Q], 
 // axial velocity (ua on axis *axis).
 template <class L, class S, bool FILM>
 __device__ __forceinline__ void color_zou_he_gather(const Grid& g, const Film& film, const ZouHe& z, const uint32_t k,
-                                                    const typename S::T* __restrict__ fin, uint32_t& i,
+                                                    const typename S::T* fin, uint32_t& i,
                                                     typename S::R (&f0)[L::Q], typename S::R (&f1)[L::Q],
                                                     uint32_t (&nbr)[L::Q], typename S::R& dens,
                                                     typename S::R& ua, int& axis, typename S::R rho_bar)
@@ -699,7 +699,7 @@ __device__ __forceinline__ void color_zou_he_gather(const Grid& g, const Film& f
 // Boundary phase pass: phi of the boundary nodes from their rebuilt populations.
 template <class L, class S, bool FILM>
 __global__ void __launch_bounds__(128)
-color_zou_he_phase(const Grid g, const Film film, const ZouHe z, const typename S::T* __restrict__ fin,
+color_zou_he_phase(const Grid g, const Film film, const ZouHe z, const typename S::T* fin,
                    double* __restrict__ phid, uint32_t* __restrict__ err, const double rho_bar)
 {
     using R = typename S::R;
@@ -732,8 +732,8 @@ template <class L, class S, int COLL, bool FILM>
 __global__ void __launch_bounds__(128)
 color_zou_he_collide(const Grid g, const Film film, const Force F, const ColorParams P, const ColorWall W,
                      const ZouHe z,
-                     const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
-                     const double* __restrict__ phid, Macros mo, const int out, uint32_t* __restrict__ err)
+                     const typename S::T* fin, typename S::T* __restrict__ fout,
+                     const double* phid, Macros mo, const int out, uint32_t* __restrict__ err)
 {
     using R = typename S::R;
     pdl_trigger();
@@ -767,7 +767,7 @@ color_zou_he_collide(const Grid g, const Film film, const Force F, const ColorPa
 // reference's initial calcMacroVar covers PB/VB).
 template <class L, class S>
 __global__ void __launch_bounds__(128)
-color_zou_he_record(const Grid g, const ZouHe z, const typename S::T* __restrict__ fin, const double rho_bar)
+color_zou_he_record(const Grid g, const ZouHe z, const typename S::T* fin, const double rho_bar)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= z.n) return;

@@ -58,7 +58,7 @@ __device__ __forceinline__ size_t idx(const Dims& d, int z, int y, int x)
 }
 
 // First statement of every kernel: let the next one be scheduled, and wait for
-// the previous ones' results.
+// the previous ones' results, which are read by plain loads (see pdl_wait).
 __device__ __forceinline__ void pdl_begin()
 {
     lbf::pdl_trigger();
@@ -85,8 +85,8 @@ __global__ void setup_fine(Dims d, const double* __restrict__ mob, double g, dou
 
 // sum_faces M_f (x_nb - x_i), and the diagonal -sum_faces M_f.
 template <class T>
-__device__ __forceinline__ T stencil(const Dims& d, const T* x, const float* __restrict__ mx,
-                                     const float* __restrict__ my, const float* __restrict__ mz, size_t i, int z,
+__device__ __forceinline__ T stencil(const Dims& d, const T* x, const float* mx,
+                                     const float* my, const float* mz, size_t i, int z,
                                      int y, int xx, T& diag)
 {
     const size_t xm = idx(d, z, y, wrapi(xx - 1, d.nx)), xp = idx(d, z, y, wrapi(xx + 1, d.nx));
@@ -100,8 +100,8 @@ __device__ __forceinline__ T stencil(const Dims& d, const T* x, const float* __r
 }
 
 // The diagonal alone, as stencil() forms it.
-__device__ __forceinline__ float diagonal(const Dims& d, const float* __restrict__ mx, const float* __restrict__ my,
-                                          const float* __restrict__ mz, size_t i, int z, int y, int xx)
+__device__ __forceinline__ float diagonal(const Dims& d, const float* mx, const float* my,
+                                          const float* mz, size_t i, int z, int y, int xx)
 {
     const float a = mx[i], b = mx[idx(d, z, y, wrapi(xx - 1, d.nx))], e = my[i],
                 f = my[idx(d, z, wrapi(y - 1, d.ny), xx)], gg = mz[i], k = mz[idx(d, wrapi(z - 1, d.nz), y, xx)];
@@ -109,8 +109,8 @@ __device__ __forceinline__ float diagonal(const Dims& d, const float* __restrict
 }
 
 // One damped Jacobi sweep: xo = xi + omega (r - A xi) / diag   (FP32)
-__global__ void jacobi(Dims d, float h2inv, float omega, const float* __restrict__ xi, const float* __restrict__ r,
-                       const float* __restrict__ mx, const float* __restrict__ my, const float* __restrict__ mz,
+__global__ void jacobi(Dims d, float h2inv, float omega, const float* xi, const float* r,
+                       const float* mx, const float* my, const float* mz,
                        float* __restrict__ xo)
 {
     pdl_begin();
@@ -124,8 +124,8 @@ __global__ void jacobi(Dims d, float h2inv, float omega, const float* __restrict
 }
 
 // The first sweep, from x = 0.
-__global__ void jacobi_first(Dims d, float h2inv, float omega, const float* __restrict__ r,
-                             const float* __restrict__ mx, const float* __restrict__ my, const float* __restrict__ mz,
+__global__ void jacobi_first(Dims d, float h2inv, float omega, const float* r,
+                             const float* mx, const float* my, const float* mz,
                              float* __restrict__ xo)
 {
     pdl_begin();
@@ -138,8 +138,8 @@ __global__ void jacobi_first(Dims d, float h2inv, float omega, const float* __re
 }
 
 // res = r - A x  (FP32)
-__global__ void residual(Dims d, float h2inv, const float* __restrict__ x, const float* __restrict__ r,
-                         const float* __restrict__ mx, const float* __restrict__ my, const float* __restrict__ mz,
+__global__ void residual(Dims d, float h2inv, const float* x, const float* r,
+                         const float* mx, const float* my, const float* mz,
                          float* __restrict__ res)
 {
     pdl_begin();
@@ -152,8 +152,8 @@ __global__ void residual(Dims d, float h2inv, const float* __restrict__ x, const
 }
 
 // Coarse face mobilities: mean of the four fine faces on each coarse interface.
-__global__ void coarsen_faces(Dims c, Dims f, const float* __restrict__ fmx, const float* __restrict__ fmy,
-                              const float* __restrict__ fmz, float* __restrict__ cmx, float* __restrict__ cmy,
+__global__ void coarsen_faces(Dims c, Dims f, const float* fmx, const float* fmy,
+                              const float* fmz, float* __restrict__ cmx, float* __restrict__ cmy,
                               float* __restrict__ cmz)
 {
     pdl_begin();
@@ -194,7 +194,7 @@ __device__ __forceinline__ float restricted(const Dims& c, const Dims& f, const 
     }
     return s;
 }
-__global__ void restrict3(Dims c, Dims f, const float* __restrict__ rf, float* __restrict__ rc)
+__global__ void restrict3(Dims c, Dims f, const float* rf, float* __restrict__ rc)
 {
     pdl_begin();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -218,7 +218,7 @@ __device__ __forceinline__ float prolonged(const Dims& f, const Dims& c, const f
             for (int e = 0; e < 2; ++e) s += w[a] * w[b] * w[e] * ec[idx(c, cz[a], cy[b], cx[e])];
     return s;
 }
-__global__ void prolong_add(Dims f, Dims c, const float* __restrict__ ec, float* __restrict__ xf)
+__global__ void prolong_add(Dims f, Dims c, const float* ec, float* __restrict__ xf)
 {
     pdl_begin();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -232,8 +232,8 @@ __global__ void prolong_add(Dims f, Dims c, const float* __restrict__ ec, float*
 // of xs alternate, one barrier a sweep, of the warps that hold cells only: 120
 // sweeps on 6^3 cells took 36 us with 1,024 threads, two barriers and the
 // faces read from memory in every sweep.
-__device__ float coarse_sweeps(const Dims& d, float h2inv, int sweeps, float r, const float* __restrict__ mx,
-                               const float* __restrict__ my, const float* __restrict__ mz, float* xs, float* red)
+__device__ float coarse_sweeps(const Dims& d, float h2inv, int sweeps, float r, const float* mx,
+                               const float* my, const float* mz, float* xs, float* red)
 {
     const int n = (int)d.n(), t = threadIdx.x;
     const int nwarps = (n + 31) / 32;
@@ -281,9 +281,9 @@ __device__ float coarse_sweeps(const Dims& d, float h2inv, int sweeps, float r, 
     return x - mean(in ? x : 0.f);
 }
 
-__global__ void __launch_bounds__(1024) coarse_solve(Dims d, float h2inv, int sweeps, const float* __restrict__ r,
-                                                     const float* __restrict__ mx, const float* __restrict__ my,
-                                                     const float* __restrict__ mz, float* __restrict__ x)
+__global__ void __launch_bounds__(1024) coarse_solve(Dims d, float h2inv, int sweeps, const float* r,
+                                                     const float* mx, const float* my,
+                                                     const float* mz, float* __restrict__ x)
 {
     pdl_begin();
     __shared__ float xs[2048], red[33];
@@ -299,9 +299,9 @@ constexpr int kBottomCells = 4096;
 constexpr size_t kBottomShared = (3 * kBottomCells + 1024) * sizeof(float);
 
 __global__ void __launch_bounds__(1024)
-bottom_cycle(Dims d, float h2inv, float omega, const float* __restrict__ r, const float* __restrict__ mx,
-             const float* __restrict__ my, const float* __restrict__ mz, float* __restrict__ x, Dims c, float ch2inv,
-             int sweeps, const float* __restrict__ cmx, const float* __restrict__ cmy, const float* __restrict__ cmz)
+bottom_cycle(Dims d, float h2inv, float omega, const float* r, const float* mx,
+             const float* my, const float* mz, float* __restrict__ x, Dims c, float ch2inv,
+             int sweeps, const float* cmx, const float* cmy, const float* cmz)
 {
     pdl_begin();
     extern __shared__ float sm[];
@@ -346,15 +346,15 @@ bottom_cycle(Dims d, float h2inv, float omega, const float* __restrict__ r, cons
 }
 
 // p = the V-cycle's result (the first search direction).
-__global__ void to_f64(size_t n, const float* __restrict__ a, double* __restrict__ b)
+__global__ void to_f64(size_t n, const float* a, double* __restrict__ b)
 {
     pdl_begin();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (i < n) b[i] = (double)a[i];
 }
 // p = z + (num / den) p
-__global__ void xpby_ratio(size_t n, const float* __restrict__ z, const double* __restrict__ num,
-                           const double* __restrict__ den, double* __restrict__ p)
+__global__ void xpby_ratio(size_t n, const float* z, const double* num,
+                           const double* den, double* __restrict__ p)
 {
     pdl_begin();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -400,7 +400,7 @@ __device__ __forceinline__ void reduce_sum(size_t n, V&& value, double* __restri
 }
 
 // sum a (b null), or a . b with b the FP32 vector's values.
-__global__ void __launch_bounds__(kT) dot(size_t n, const double* __restrict__ a, const float* __restrict__ b,
+__global__ void __launch_bounds__(kT) dot(size_t n, const double* a, const float* b,
                                           double* __restrict__ part, uint32_t* __restrict__ done,
                                           double* __restrict__ out)
 {
@@ -409,8 +409,8 @@ __global__ void __launch_bounds__(kT) dot(size_t n, const double* __restrict__ a
 }
 
 // r = rhs - mean (phi = 0), its FP32 copy and r . r
-__global__ void __launch_bounds__(kT) start_dot(size_t n, const double* __restrict__ sum,
-                                                const double* __restrict__ rhs, double* __restrict__ r,
+__global__ void __launch_bounds__(kT) start_dot(size_t n, const double* sum,
+                                                const double* rhs, double* __restrict__ r,
                                                 float* __restrict__ r32, double* __restrict__ part,
                                                 uint32_t* __restrict__ done, double* __restrict__ rr)
 {
@@ -425,9 +425,9 @@ __global__ void __launch_bounds__(kT) start_dot(size_t n, const double* __restri
 }
 
 // out = A p  (FP64, the CG operator) and p . out
-__global__ void __launch_bounds__(kT) apply_dot(Dims d, double h2inv, const double* __restrict__ p,
-                                                const float* __restrict__ mx, const float* __restrict__ my,
-                                                const float* __restrict__ mz, double* __restrict__ out,
+__global__ void __launch_bounds__(kT) apply_dot(Dims d, double h2inv, const double* p,
+                                                const float* mx, const float* my,
+                                                const float* mz, double* __restrict__ out,
                                                 double* __restrict__ part, uint32_t* __restrict__ done,
                                                 double* __restrict__ pap)
 {
@@ -443,9 +443,9 @@ __global__ void __launch_bounds__(kT) apply_dot(Dims d, double h2inv, const doub
 }
 
 // phi += (rz / pap) p, r -= (rz / pap) Ap, r's FP32 copy and r . r
-__global__ void __launch_bounds__(kT) update_dot(size_t n, const double* __restrict__ rz,
-                                                 const double* __restrict__ pap, const double* __restrict__ p,
-                                                 const double* __restrict__ Ap, double* __restrict__ phi,
+__global__ void __launch_bounds__(kT) update_dot(size_t n, const double* rz,
+                                                 const double* pap, const double* p,
+                                                 const double* Ap, double* __restrict__ phi,
                                                  double* __restrict__ r, float* __restrict__ r32,
                                                  double* __restrict__ part, uint32_t* __restrict__ done,
                                                  double* __restrict__ rr)
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(kT) update_dot(size_t n, const double* __restr
     }, part, done, rr);
 }
 
-__global__ void sub_mean(size_t n, const double* __restrict__ sum, double* __restrict__ a)
+__global__ void sub_mean(size_t n, const double* sum, double* __restrict__ a)
 {
     pdl_begin();
     const size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;

@@ -64,6 +64,11 @@ struct Macros {                 // compact per-node outputs, stride nfp
 // previous kernels of the stream to complete and be visible.  The launch gap,
 // the occupancy lookups and the previous step's last, partly filled round of
 // blocks then overlap.  Both are no-ops in a kernel launched without it.
+// What earlier kernels write (populations, exponents, phase field, densities)
+// changes within the lifetime of a kernel that starts early, so it is read
+// behind the wait by plain loads, through pointers that are not `const
+// __restrict__`: the read-only path is for data that stays the same throughout,
+// and its loads need not stay behind the wait.
 // Microseconds per step without -> with: FP64 48^3 (24 k nodes) 6.2 -> 4.8,
 // 96^3 12.4 -> 9.5, 256^3 (3.7 M) 186.8 -> 184.1; FP16 192^3 51.1 -> 48.3.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -91,7 +96,7 @@ struct StoreF64 {
     using T = double;
     using R = double;
     static constexpr bool shifted = false;
-    __device__ static R load(const T* p, int, R) { return __ldg(p); }
+    __device__ static R load(const T* p, int, R) { return *p; }
     __device__ static void store(T* p, R v, int, R) { *p = v; }
 };
 // Shifted deviations g_q = f_q - w_q rho0, stored as h_q = g_q * (4096 / w_q)
@@ -151,7 +156,7 @@ template <class L, class H> struct StoreShifted16 {
     // and the batched step -- computes bitwise the same fields.
     __device__ static R load(const T* p, int q, R)
     {
-        return __fmul_rn(float(__ldg(p)), ShiftScale<L>::inv(q));
+        return __fmul_rn(float(*p), ShiftScale<L>::inv(q));
     }
     // The value that load() gives for these stored bits.
     __device__ static R from_bits(uint16_t b, int q)
@@ -201,7 +206,7 @@ template <class L> struct StoreF32 {
     using T = float;
     using R = float;
     static constexpr bool shifted = true;
-    __device__ static R load(const T* p, int, R) { return __ldg(p); }
+    __device__ static R load(const T* p, int, R) { return *p; }
     __device__ static void store(T* p, R v, int, R) { *p = v; }
 };
 
@@ -212,7 +217,7 @@ struct StoreF32Full {
     using T = float;
     using R = float;
     static constexpr bool shifted = false;
-    __device__ static R load(const T* p, int, R) { return __ldg(p); }
+    __device__ static R load(const T* p, int, R) { return *p; }
     __device__ static void store(T* p, R v, int, R) { *p = v; }
 };
 
@@ -233,7 +238,7 @@ template <class L> struct StoreBFP16 {
     __device__ static R load(const T*, int, R) { return R(0); }
     __device__ static void store(T*, R, int, R) {}
     __device__ static R load_blk(const T* p, int q, int e)
-    { return (float)__ldg(p) * (pow2f(e - 15) * ((float)L::w36f(q) / 36.0f)); }
+    { return (float)*p * (pow2f(e - 15) * ((float)L::w36f(q) / 36.0f)); }
     // Exponent of a node whose largest |x_q| is m.
     __device__ static int exponent(float m)
     {
@@ -269,9 +274,9 @@ template <class L> struct StoreBFP16 {
 // voxel x + e_q (the pull source of op q) or UINT32_MAX when it is solid.
 template <class S>
 __device__ __forceinline__ typename S::R load_pop(const typename S::T* p, int q, typename S::R rho0,
-                                                  const int8_t* __restrict__ ein, uint32_t src)
+                                                  const int8_t* ein, uint32_t src)
 {
-    if constexpr (S::blocked) return S::load_blk(p, q, (int)__ldg(&ein[src]));
+    if constexpr (S::blocked) return S::load_blk(p, q, (int)ein[src]);
     else return S::load(p, q, rho0);
 }
 
@@ -463,10 +468,10 @@ build_links(const Grid g, uint4* __restrict__ row, uint32_t* __restrict__ mask, 
 }
 
 template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4), bool LINKS = false>
-__device__ __forceinline__ void gather(const Grid& g, const typename S::T* __restrict__ fin,
+__device__ __forceinline__ void gather(const Grid& g, const typename S::T* fin,
                                        uint32_t i, int x, int y, int z,
                                        typename S::R (&f)[L::Q], uint32_t (&nbr)[L::Q],
-                                       typename S::R rho0, const int8_t* __restrict__ ein = nullptr,
+                                       typename S::R rho0, const int8_t* ein = nullptr,
                                        const Links& links = Links{})
 {
     // Element offsets stay 32-bit (phases * Q * nfp < 2^32 is checked at
@@ -729,10 +734,10 @@ __device__ __forceinline__ void scsp_store(const Grid& g, const ScspParams& P, t
 // kernel).
 template <class L, class S, bool PULL, bool UNIFORM = (sizeof(typename S::R) == 4), bool LINKS = false>
 __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const ScspParams& P,
-                                            const typename S::T* __restrict__ fin,
+                                            const typename S::T* fin,
                                             typename S::T* __restrict__ fout, const uint32_t i,
                                             const Macros& mo, const int out, uint32_t* __restrict__ err,
-                                            const int8_t* __restrict__ ein, int8_t* __restrict__ eout,
+                                            const int8_t* ein, int8_t* __restrict__ eout,
                                             const Links& links = Links{})
 {
     int x = 0, y = 0, z = 0;
@@ -857,9 +862,9 @@ __device__ __forceinline__ typename S::R zou_he_node(typename S::R (&f)[L::Q], u
 // Update of the k-th boundary node.
 template <class L, class S>
 __device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, const ZouHe& z, const uint32_t k,
-                                         const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+                                         const typename S::T* fin, typename S::T* __restrict__ fout,
                                          const Macros& mo, const int out, uint32_t* __restrict__ err,
-                                         const int8_t* __restrict__ ein, int8_t* __restrict__ eout)
+                                         const int8_t* ein, int8_t* __restrict__ eout)
 {
     using R = typename S::R;
     const uint32_t i = __ldg(&z.node[k]);
@@ -957,9 +962,9 @@ __device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, 
 template <class L, class S, bool PULL, bool BOUNDARY, bool LINKS>
 __global__ void __launch_bounds__(128, BOUNDARY ? StepBlocks<S>::boundary : StepBlocks<S>::value)
 scsp_step(const Grid g, const Force F, const ScspParams P,
-          const typename S::T* __restrict__ fin, typename S::T* __restrict__ fout,
+          const typename S::T* fin, typename S::T* __restrict__ fout,
           Macros mo, const int out, uint32_t* __restrict__ err,
-          const int8_t* __restrict__ ein, int8_t* __restrict__ eout, const ZouHe z, const uint32_t zblocks,
+          const int8_t* ein, int8_t* __restrict__ eout, const ZouHe z, const uint32_t zblocks,
           const Links links)
 {
     // The node order alternates between steps: a step that runs in the

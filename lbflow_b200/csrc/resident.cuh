@@ -135,7 +135,7 @@ __device__ __forceinline__ bool resident_late(long long& t0, uint32_t* err)
 // step's rounding seed follows as in the one-step launches.
 template <class L, class S>
 __global__ void __launch_bounds__(kResidentThreads, ResidentBlocks<L, S>::value)
-scsp_resident(const Grid g, const Force F, const ScspParams P0, const typename S::T* __restrict__ fin,
+scsp_resident(const Grid g, const Force F, const ScspParams P0, const typename S::T* fin,
               typename S::T* __restrict__ fout, const Resident r, Macros mo, const int out,
               uint32_t* __restrict__ err)
 {
