@@ -458,10 +458,14 @@ __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constan
 // shared memory where they are few, else they stream through a ring of `stages`
 // slots of `per` taps (a slot per tap is bound by the latency of its refill);
 // each is used by the kCZ z slices' accumulators.  The K order per output is
-// igemm's (tap, then channel).
+// igemm's (tap, then channel), 16 at a time, so the result is too, bit for bit:
+// channel counts that are a multiple of 16, and 8, where a K step takes two
+// taps, one in each half (the halves of an operand lie any distance apart; 8 ->
+// 16 at 96^3 33 us, 45 with a half of zeros beside each tap).  Other counts
+// split a tap's channels over K steps and stay with igemm.
 //
 // Measured, igemm -> here: 16 -> 16 channels at 96^3 238 -> 48 us, 8 -> 16 187
-// -> 44, 32 -> 16 (two sources) 403 -> 102, 32 -> 32 at 48^3 63 -> 22, 64 -> 64
+// -> 33, 32 -> 16 (two sources) 403 -> 102, 32 -> 32 at 48^3 63 -> 22, 64 -> 64
 // at 2 x 48^3 91 -> 82.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
 // (cp.async at 14 bytes a cycle), 28,000 for 432 MMAs (N = 64, 65 cycles each;
 // operand reads alone need 48), the rest weights and epilogue.  Narrow inputs
@@ -480,14 +484,20 @@ constexpr int kConvProducers = 256, kConvThreads = kConvProducers + 32;
 constexpr uint32_t kMaxConvC = 64;
 struct TapRing { uint32_t per, stages; };
 
+// Taps held with G channel groups: a 28th of zero weights completes the last
+// pair of a single group, whose operand half then reads kZeros bytes of zeros.
+constexpr uint32_t conv_taps(uint32_t groups) { return groups == 1 ? 28 : 27; }
+constexpr uint32_t kZeros = ((kCY - 1) * kHX + 8) * 16;
+
 constexpr size_t conv3_smem(uint32_t groups, uint32_t bn, TapRing r) {
-    return 128 + size_t(groups) * kPlane + size_t(r.per) * r.stages * groups * bn * 16 + (2 + 2 * kTapStages) * 8 + 16;
+    return 128 + size_t(groups) * kPlane + size_t(r.per) * r.stages * groups * bn * 16 + (groups == 1 ? kZeros : 0) +
+           (2 + 2 * kTapStages) * 8 + 16;
 }
 
-// G: 8-channel groups held (2, 4 or 8; those past the input's channels are
+// G: 8-channel groups held (1, 2, 4 or 8; those past the input's channels are
 // zeros).
 template <int BN, int G>
-__global__ void __launch_bounds__(kConvThreads, G == 2 ? 4 : (G == 4 ? 2 : 1))
+__global__ void __launch_bounds__(kConvThreads, G <= 2 ? 4 : (G == 4 ? 2 : 1))
 conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint32_t ty, const uint32_t tz,
              const TapRing ring) {
     extern __shared__ uint8_t smem_raw[];
@@ -496,7 +506,8 @@ conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint3
     const uint32_t a0 = (smem_u32(smem_raw) + 127u) & ~127u;
     const uint32_t w0 = a0 + G * kPlane;
     const uint32_t slot_bytes = ring.per * tap_bytes;
-    const uint32_t bar = (w0 + ring.stages * slot_bytes + 7u) & ~7u;
+    const uint32_t zeros = w0 + ring.stages * slot_bytes;
+    const uint32_t bar = (zeros + (G == 1 ? kZeros : 0u) + 7u) & ~7u;
     const uint32_t full_a = bar, done = bar + 8u, full0 = bar + 16u, empty0 = full0 + kTapStages * 8u;
     const uint32_t slot = empty0 + kTapStages * 8u;
 
@@ -558,9 +569,10 @@ conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint3
 #pragma unroll
             for (int i = 0; i < kHX; ++i) cp_async16(dst + i * 16u, row + xo[i], bytes);
         }
+        if (G == 1 && threadIdx.x < kZeros / 16u) cp_async16(zeros + threadIdx.x * 16u, p.g.src0, 0u);
         cp_async_arrive(full_a);
         const uint16_t* const wp = in ? p.w + size_t(n0) * p.k_pad + ch : p.w;
-        const uint32_t total = 27u / ring.per;
+        const uint32_t total = conv_taps(G) / ring.per;
         for (uint32_t st = 0; st < total; ++st) {
             const uint32_t s = st % ring.stages;
             if (st >= ring.stages) {
@@ -570,8 +582,9 @@ conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint3
             }
             for (uint32_t q = first; q < ring.per * BN; q += kStep) {
                 const uint32_t tap = q / BN, n = q % BN;
+                const bool real = in && st * ring.per + tap < 27u;
                 cp_async16(w0 + s * slot_bytes + tap * tap_bytes + (g8 * BN + n) * 16u,
-                           in ? wp + n * p.k_pad + (st * ring.per + tap) * p.g.ct : wp, bytes);
+                           real ? wp + n * p.k_pad + (st * ring.per + tap) * p.g.ct : p.w, real ? 16u : 0u);
             }
             cp_async_arrive(full0 + 8u * s);
         }
@@ -588,21 +601,37 @@ conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint3
         // Descriptors differ in their start address (16-byte units) only.
         const uint64_t ad0 = desc_plain(a0, kPlane, kHX * 16u);
         const uint64_t bd0 = desc_plain(w0, BN * 16u, 128u);
-        for (uint32_t st = 0; st < 27u / ring.per && go; ++st) {
+        for (uint32_t st = 0; st < conv_taps(G) / ring.per && go; ++st) {
             const uint32_t s = st % ring.stages;
             go = __all_sync(0xffffffffu, mbar_wait(full0 + 8u * s, (st / ring.stages) & 1u, kWaitCycles));
             if (!go) break;
             fence_async_shared();
             fence_after_sync();
-            for (uint32_t j = 0; j < ring.per; ++j) {
-                const uint32_t tap = st * ring.per + j;
-                const uint32_t dz = tap / 9u, dy = tap / 3u - 3u * dz, dx = tap % 3u;
-                uint64_t ad = ad0 + (dz * kHY + dy) * kHX + dx;
-                uint64_t bd = bd0 + (s * slot_bytes + j * tap_bytes) / 16u;
-                for (uint32_t k = 0; k < uint32_t(G); k += 2, ad += 2 * kPlane / 16u, bd += 2 * BN)
+            if constexpr (G == 1) {
+                // Taps 2 j and 2 j + 1 in one K step, the distance between them as
+                // the distance between the operand's K halves.
+                auto voxel = [](uint32_t tap) { return (tap / 9u * kHY + tap / 3u % 3u) * kHX + tap % 3u; };
+                const uint64_t plain = desc_plain(a0, 0u, kHX * 16u);
+                for (uint32_t j = 0; j < conv_taps(G) / 2u; ++j) {
+                    const uint32_t at = voxel(2u * j), bd = 2u * j * BN;
 #pragma unroll
-                    for (uint32_t z = 0; z < uint32_t(kCZ); ++z)
-                        mma_bf16_warp(leader, tmem + z * BN, ad + z * (kHX * kHY), bd, idesc, (tap | k) != 0u);
+                    for (uint32_t z = 0; z < uint32_t(kCZ); ++z) {
+                        const uint32_t from = at + z * (kHX * kHY);
+                        const uint32_t apart = 2u * j + 1u < 27u ? voxel(2u * j + 1u) - at : (zeros - a0) / 16u - from;
+                        mma_bf16_warp(leader, tmem + z * BN, plain + from + (uint64_t(apart) << 16), bd0 + bd, idesc, j != 0u);
+                    }
+                }
+            } else {
+                for (uint32_t j = 0; j < ring.per; ++j) {
+                    const uint32_t tap = st * ring.per + j;
+                    const uint32_t dz = tap / 9u, dy = tap / 3u - 3u * dz, dx = tap % 3u;
+                    uint64_t ad = ad0 + (dz * kHY + dy) * kHX + dx;
+                    uint64_t bd = bd0 + (s * slot_bytes + j * tap_bytes) / 16u;
+                    for (uint32_t k = 0; k < uint32_t(G); k += 2, ad += 2 * kPlane / 16u, bd += 2 * BN)
+#pragma unroll
+                        for (uint32_t z = 0; z < uint32_t(kCZ); ++z)
+                            mma_bf16_warp(leader, tmem + z * BN, ad + z * (kHX * kHY), bd, idesc, (tap | k) != 0u);
+                }
             }
             commit_warp(leader, empty0 + 8u * s);
         }
@@ -995,11 +1024,12 @@ int launch_igemm(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
 }
 
 // Whether conv3_kernel takes the call: a 3x3x3 periodic convolution of at most
-// kMaxConvC channels into rows, whose tiles are not mostly padding.
+// kMaxConvC channels, 8 or a multiple of 16, into rows, whose tiles are not
+// mostly padding.
 bool conv3_fits(const IgemmArgs& p) {
     const Gather& g = p.g;
-    if (g.ks != 3 || g.stride != 1 || g.pad != 1 || g.ct > kMaxConvC || p.mode == LBF_OUT_SCATTER2_BF16 ||
-        g.in_d != g.out_d || g.in_h != g.out_h || g.in_w != g.out_w)
+    if (g.ks != 3 || g.stride != 1 || g.pad != 1 || g.ct > kMaxConvC || (g.ct != 8 && g.ct % 16 != 0) ||
+        p.mode == LBF_OUT_SCATTER2_BF16 || g.in_d != g.out_d || g.in_h != g.out_h || g.in_w != g.out_w)
         return false;
     auto up = [](uint64_t n, uint64_t t) { return (n + t - 1) / t * t; };
     return up(g.out_w, kCX) * up(g.out_h, kCY) * up(g.out_d, kCZ) <= 2ull * g.out_w * g.out_h * g.out_d;
@@ -1011,8 +1041,8 @@ template <int BN, int G>
 int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
     // All 27 taps' weights where that leaves room for three blocks on an SM, else
     // three slots of as many taps as fit into one block's shared memory.
-    TapRing ring{27, 1};
-    if (conv3_smem(G, BN, ring) > kSmemMost / 3) ring = TapRing{3, 3};
+    TapRing ring{conv_taps(G), 1};
+    if (G > 1 && conv3_smem(G, BN, ring) > kSmemMost / 3) ring = TapRing{3, 3};
     if (conv3_smem(G, BN, ring) > kSmemMost) ring = TapRing{1, 3};
     const size_t sm = conv3_smem(G, BN, ring);
     cudaError_t e = cudaFuncSetAttribute(conv3_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
@@ -1028,6 +1058,7 @@ int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
 
 template <int BN>
 int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
+    if (p.g.ct == 8) return launch_conv3<BN, 1>(p, n_pad, s);
     return p.g.ct <= 16 ? launch_conv3<BN, 2>(p, n_pad, s)
                         : (p.g.ct <= 32 ? launch_conv3<BN, 4>(p, n_pad, s) : launch_conv3<BN, 8>(p, n_pad, s));
 }
