@@ -465,8 +465,8 @@ __global__ void __launch_bounds__(kThreads, 1) igemm_kernel(const __grid_constan
 // split a tap's channels over K steps and stay with igemm.
 //
 // Measured, igemm -> here: 16 -> 16 channels at 96^3 238 -> 48 us, 8 -> 16 187
-// -> 33, 32 -> 16 (two sources) 403 -> 102, 32 -> 32 at 48^3 63 -> 22, 64 -> 64
-// at 2 x 48^3 91 -> 82.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
+// -> 33, 32 -> 16 (two sources) 403 -> 102, 32 -> 32 at 48^3 63 -> 22, 32 + 32
+// -> 64 at 2 x 48^3 213 -> 80.  Per 64-channel block of 52,000 cycles: 10,000 for the halo
 // (cp.async at 14 bytes a cycle), 28,000 for 432 MMAs (N = 64, 65 cycles each;
 // operand reads alone need 48), the rest weights and epilogue.  Narrow inputs
 // need several resident blocks to overlap those phases: the registers are
@@ -1025,10 +1025,14 @@ int launch_igemm(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
 
 // Whether conv3_kernel takes the call: a 3x3x3 periodic convolution of at most
 // kMaxConvC channels, 8 or a multiple of 16, into rows, whose tiles are not
-// mostly padding.
+// mostly padding.  64 channels of one source stay with igemm, which fetches a
+// row's 128 bytes as one piece then: 64 -> 64 at 24^3 x 2 22 us, 27 here, at 36 x
+// 48 x 48 42 and 51, at 48^3 x 2 81 and 82, at 96^3 304 and 302.  From two sources
+// (32 + 32 -> 32 at 48^3 x 2 201 us, 66 here) or with fewer channels (48 -> 64 170
+// and 74) it works piece by piece and loses at every size.
 bool conv3_fits(const IgemmArgs& p) {
     const Gather& g = p.g;
-    if (g.ks != 3 || g.stride != 1 || g.pad != 1 || g.ct > kMaxConvC || (g.ct != 8 && g.ct % 16 != 0) ||
+    if (g.ks != 3 || g.stride != 1 || g.pad != 1 || g.ct > kMaxConvC || (g.ct != 8 && g.ct % 16 != 0) || g.c0 == kMaxConvC ||
         p.mode == LBF_OUT_SCATTER2_BF16 || g.in_d != g.out_d || g.in_h != g.out_h || g.in_w != g.out_w)
         return false;
     auto up = [](uint64_t n, uint64_t t) { return (n + t - 1) / t * t; };

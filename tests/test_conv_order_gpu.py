@@ -28,7 +28,7 @@ def _run(x0, x1, w, b, slope, f32):
     (8, 0, 16), (8, 0, 32), (8, 0, 64), (8, 0, 128), (8, 0, 200),     # two taps in a K step
     (16, 0, 16), (8, 8, 32), (16, 0, 64), (16, 0, 128),
     (32, 0, 32), (16, 16, 16), (32, 0, 64), (24, 8, 128), (48, 0, 24),
-    (64, 0, 64), (32, 32, 32), (64, 0, 128), (64, 0, 256),
+    (32, 32, 32), (48, 16, 64), (32, 32, 256),
 ])
 def test_same_bits_from_both_kernels(c0, c1, cout):
     gen = torch.Generator().manual_seed(c0 + 3 * c1 + 5 * cout)
@@ -47,9 +47,10 @@ def test_same_bits_from_both_kernels(c0, c1, cout):
         assert torch.equal(out[0][0].repeat(1, 2, 4, 1, 1), out[1][0])
 
 
-@pytest.mark.parametrize('channels', [24, 40, 56])
-def test_split_taps_stay_with_the_gathering_kernel(channels):
-    """Channel counts whose K steps straddle taps unevenly."""
+@pytest.mark.parametrize('channels', [24, 40, 56, 64])
+def test_calls_that_stay_with_the_gathering_kernel(channels):
+    """Channel counts whose K steps straddle taps unevenly, and 64 from one
+    source, whose rows that kernel fetches whole, faster at every size."""
     x = torch.randn(1, 4, 16, 16, channels, device='cuda').to(torch.bfloat16)
     w = torch.randn(16, channels, 3, 3, 3, device='cuda')
     assert _run(x, None, w, None, None, False)[1] == {'igemm_kernel'}
