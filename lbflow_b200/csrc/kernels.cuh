@@ -772,9 +772,10 @@ template <> struct StepBlocks<StoreF64> { static constexpr int value = 7, bounda
 // kernel's first blocks update the boundary nodes, one thread per node of a
 // compact list; the other blocks skip those nodes by a bitmap (one word per
 // warp).  A boundary node's update is a long dependent chain on few warps: as
-// a launch of its own after the step it left the rest of the chip idle
-// (161x93x117, 537 k nodes, two pressure planes: FP64 45.4 -> 37.4 us per
-// step, FP32 27.1 -> 16.4).
+// a launch of its own after the step it leaves the rest of the chip idle
+// (161x93x117, 537 k nodes, two pressure planes: FP64 42.2 us per step, 37.6
+// inside; FP32 23.5 and 18.7).  Large geometries keep the launch of its own
+// (zou_he_inside).
 struct ZouHe {
     uint32_t n;                          // boundary nodes
     const uint32_t* __restrict__ bits;   // single phase: bit i of the map is set when node i is one
@@ -955,6 +956,19 @@ __device__ __forceinline__ void scsp_zou_he(const Grid& g, const ScspParams& P, 
 #pragma unroll
         for (int q = 0; q < L::Q; ++q) S::store(fout + (q * g.nfp + i), f[q], q, rho0);
     }
+}
+
+// The boundary nodes in a launch of their own, after the step's (same buffers):
+// what the step stored and reported for them is overwritten.
+template <class L, class S>
+__global__ void __launch_bounds__(128)
+scsp_zou_he_pass(const Grid g, const ScspParams P, const ZouHe z, const typename S::T* fin,
+                 typename S::T* __restrict__ fout, Macros mo, const int out, uint32_t* __restrict__ err,
+                 const int8_t* ein, int8_t* __restrict__ eout)
+{
+    pdl_trigger();
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < z.n) scsp_zou_he<L, S>(g, P, z, k, fin, fout, mo, out, err, ein, eout);
 }
 
 // One step of every node.  BOUNDARY: the grid's first `zblocks` blocks update

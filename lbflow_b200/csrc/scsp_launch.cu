@@ -10,6 +10,26 @@ template <class L, class S> struct UseLinks {
     static constexpr bool value = L::D == 3 && sizeof(typename S::T) == 2;
 };
 
+// Whether the step's launch updates the nb boundary nodes too; otherwise a launch
+// of their own follows it.  Inside, their chain overlaps with the other nodes'
+// work, but FP64 then runs the whole step at five blocks per SM instead of seven,
+// and a boundary node's populations, written apart from their neighbours', leave
+// sectors that large geometries write back and read in parts.  Inside / apart, us
+// per step (nodes, boundary nodes):
+//   FP64  537 k, 21 k 37.6 / 42.2;  482 k, 44 k 41.5 / 43.7;  865 k, 8 k 52.4 /
+//         54.0;  894 k, 19 k 60.6 / 60.5;  671 k, 78 k 70.6 / 65.9;  1.73 M, 8 k
+//         103 / 96;  2.5 M, 78 k 199 / 174;  5.1 M, 129 k 396 / 341
+//   FP32  537 k, 21 k 18.7 / 23.5;  1.05 M, 44 k 47.9 / 49.7;  2.9 M, 19 k 99.0 /
+//         102.4;  783 k, 178 k 44.5 / 45.6;  1.52 M, 56 k 74.5 / 72.2;  2.5 M, 78 k
+//         125 / 117;  5.1 M, 129 k 247 / 228;  10 M, 28 k 321 / 309
+//   FP16  537 k, 21 k 15.3 / 27.1;  5.1 M, 129 k 189 / 227;  3.5 M, 317 k 148 / 188
+template <class S> bool zou_he_inside(uint64_t nf, uint64_t nb)
+{
+    if constexpr (sizeof(typename S::T) == 8) return nf + 8 * nb <= 950000;
+    if constexpr (sizeof(typename S::T) == 4) return nf * nb <= 80000000000ull;
+    return true;
+}
+
 template <class L, class S>
 void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
 {
@@ -21,7 +41,8 @@ void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
     (void)mrt;   // the collision rates (SRT or MRT) are in a.P.rate
     // At t = 0 (no pull) the boundary nodes hold rho0 at rest, which the
     // ordinary update reproduces from their initial populations.
-    const unsigned zb = pull ? blocks_for(a.zh.n, threads) : 0;
+    const unsigned zall = pull ? blocks_for(a.zh.n, threads) : 0;
+    const unsigned zb = zou_he_inside<S>(a.g.nf, a.zh.n) ? zall : 0;
     auto step = [&](auto kernel) {
         launch_pdl(kernel, zb + blocks, threads, a.stream, a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout,
                    a.zh, zb, a.links);
@@ -31,15 +52,22 @@ void dispatch(bool mrt, bool pull, int out, const ScspLaunch& a)
             a.g, a.F, a.P, fin, fout, a.mo, out, a.err, a.ein, a.eout, a.zh, 0u, a.links);
         return;
     }
+    bool done = false;
     if constexpr (UseLinks<L, S>::value) {
         if (a.links.row) {
             if (zb) step(scsp_step<L, S, true, true, true>);
             else step(scsp_step<L, S, true, false, true>);
-            return;
+            done = true;
         }
     }
-    if (zb) step(scsp_step<L, S, true, true, false>);
-    else step(scsp_step<L, S, true, false, false>);
+    if (!done) {
+        if (zb) step(scsp_step<L, S, true, true, false>);
+        else step(scsp_step<L, S, true, false, false>);
+    }
+    if constexpr (sizeof(T) >= 4)
+        if (zall && !zb)
+            launch_pdl(scsp_zou_he_pass<L, S>, zall, threads, a.stream, a.g, a.P, a.zh, fin, fout, a.mo, a.out, a.err,
+                       a.ein, a.eout);
 }
 
 template <class L>
