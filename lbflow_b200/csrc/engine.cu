@@ -942,24 +942,8 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
         LBF_ALLOC(e->link_row, tiles * kLinkTile);
         LBF_ALLOC(e->link_mask, tiles * kLinkTile);
         LBF_ALLOC(e->link_base, 2 * tiles);
-        // d_used has been read: its first word counts the nodes without offsets.
-        LBF_CUDA(cudaMemsetAsync(d_used, 0, sizeof(uint32_t), e->stream));
-        launch_build_links(grid_of(e), e->link_row, e->link_mask, e->link_base, d_used, e->stream);
+        launch_build_links(grid_of(e), e->link_row, e->link_mask, e->link_base, e->stream);
         LBF_CUDA(cudaGetLastError());
-        uint32_t none = 0;
-        LBF_CUDA(cudaMemcpyAsync(e->h_red, d_used, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->stream));
-        LBF_CUDA(cudaStreamSynchronize(e->stream));
-        std::memcpy(&none, e->h_red, sizeof none);
-        // Planes of more than about 65,000 fluid nodes overflow everywhere: the
-        // lookups alone are then the faster form.
-        if (none > e->nf / 16) {
-            cudaFreeAsync(e->link_row, e->stream);
-            cudaFreeAsync(e->link_mask, e->stream);
-            cudaFreeAsync(e->link_base, e->stream);
-            e->link_row = e->link_base = nullptr;
-            e->link_mask = nullptr;
-            e->bytes -= tiles * (kLinkTile * (sizeof(uint4) + sizeof(uint32_t)) + 2 * sizeof(uint4));
-        }
     }
     if (boundaries || c.model == LBF_MODEL_COLOR) {
         if ((rc = ensure_vox(e))) { std::string m = e->last_error; lbf_destroy(e); return fail(nullptr, rc, m); }

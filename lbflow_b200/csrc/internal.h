@@ -46,7 +46,7 @@ struct ColorLaunch {
 void launch_scsp(int dims, int storage, bool mrt, bool pull, int out, const ScspLaunch& a);
 // The table of pull sources: whether a storage's steps use it, and its fill.
 bool scsp_uses_links(int dims, int storage);
-void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, uint32_t* none, cudaStream_t s);
+void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, cudaStream_t s);
 void launch_scsp_init(int dims, int storage, const Grid& g, const Force& F, double rho0,
                       void* f, int8_t* eout, cudaStream_t s);
 // All steps of a call in one launch (resident.cuh): a.out applies to the last.

@@ -367,9 +367,11 @@ __device__ __forceinline__ uint32_t pull_sources(const Grid& g, int x, int y, in
 // (tiles of 128 consecutive nodes, the step kernel's blocks), and a word with
 // the 18 fluid bits and two marks for x = 0 and x = nx - 1, whose sources
 // beyond the wrap are looked up as before: 20 bytes per node in place of the
-// 4-byte coordinate.  A third mark sends a node to the lookups altogether:
-// one whose offsets do not fit (a tile across the end of the first or last
-// plane, whose z neighbours wrap).
+// 4-byte coordinate.  A third mark sends a node to the lookups altogether: one
+// whose offsets do not fit.  A tile's offsets exceed 16 bits where it straddles a
+// periodic wrap in y or z between planes of more than 65,536 nodes, or where a
+// neighbouring row or plane holds 512 times its nodes; either way a small part of
+// a geometry's nodes (3 x 270 x 290 voxels 0.31 %, 3 x 2048 x 2048 0.007 %).
 struct Links {
     const uint4* __restrict__ row;       // [node] eight 16-bit offsets
     const uint32_t* __restrict__ mask;   // [node] bit q: the source of q is fluid
@@ -426,11 +428,10 @@ __device__ __forceinline__ uint32_t link_sources(const Grid& g, const Links& k, 
     return m;
 }
 
-// Fills the table, one block per tile; *none counts the nodes without offsets.
+// Fills the table, one block per tile.
 template <class L>
 __global__ void __launch_bounds__(kLinkTile)
-build_links(const Grid g, uint4* __restrict__ row, uint32_t* __restrict__ mask, uint4* __restrict__ base,
-            uint32_t* __restrict__ none)
+build_links(const Grid g, uint4* __restrict__ row, uint32_t* __restrict__ mask, uint4* __restrict__ base)
 {
     __shared__ uint32_t low[8];
     const uint32_t i = blockIdx.x * kLinkTile + threadIdx.x;
@@ -453,10 +454,7 @@ build_links(const Grid g, uint4* __restrict__ row, uint32_t* __restrict__ mask, 
         uint32_t d[8], worst = 0;
 #pragma unroll
         for (int r = 0; r < 8; ++r) { d[r] = idx[r] - low[r]; worst |= d[r]; }
-        if (worst > 0xffffu) {
-            atomicAdd(none, 1u);
-            m |= kLinkNone;
-        }
+        if (worst > 0xffffu) m |= kLinkNone;
         row[i] = make_uint4((d[0] & 0xffffu) | (d[1] << 16), (d[2] & 0xffffu) | (d[3] << 16),
                             (d[4] & 0xffffu) | (d[5] << 16), (d[6] & 0xffffu) | (d[7] << 16));
         mask[i] = m;

@@ -170,10 +170,10 @@ bool scsp_uses_links(int dims, int storage)
     return dims == 3 && storage != LBF_STORE_FP64 && storage != LBF_STORE_FP32;
 }
 
-void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, uint32_t* none, cudaStream_t s)
+void launch_build_links(const Grid& g, uint4* row, uint32_t* mask, uint4* base, cudaStream_t s)
 {
     const unsigned blocks = blocks_for(g.nf, kLinkTile);
-    if (blocks) build_links<D3Q19><<<blocks, kLinkTile, 0, s>>>(g, row, mask, base, none);
+    if (blocks) build_links<D3Q19><<<blocks, kLinkTile, 0, s>>>(g, row, mask, base);
 }
 
 void launch_scsp_add_density(int dims, int storage, const Grid& g, const float* drho, void* f, int8_t* e,
