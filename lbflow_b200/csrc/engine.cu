@@ -32,8 +32,8 @@ struct lbf_engine {
     int cur = 0;
     uint2* occ = nullptr;
     uint32_t* coord = nullptr;
-    uint4 *link_row = nullptr, *link_base = nullptr;   // table of pull sources
-    uint32_t* link_mask = nullptr;
+    void* link_table = nullptr;     // memory of `links`, the table of pull sources (optional)
+    Links links{};
     uint8_t* node_label = nullptr;
     uint8_t* node_phase = nullptr;
     double* label_force = nullptr;
@@ -64,7 +64,7 @@ struct lbf_engine {
     bool initialized = false;
     uint32_t steps = 0;             // pull steps launched (seeds the 16-bit stochastic rounding)
     uint32_t pulls = 0;             // pull steps launched (alternates the step kernel's node order)
-    void* words = nullptr;          // tagged words of the resident steps (allocated on first use)
+    void* words = nullptr;          // tagged words of the resident steps (optional, allocated on first use)
     uint32_t tag = 0;               // step number of the last resident step
     bool resident_asked = false;    // resident_nodes is known
     uint32_t resident_nodes = 0;    // largest geometry the resident steps take
@@ -127,20 +127,82 @@ namespace {
 
 cudaError_t engine_pool(int device, cudaMemPool_t* pool) { return lbf::device_pool(device, pool); }
 
+// Device memory of the engine from the pool, counted in e->bytes.
+cudaError_t pool_alloc(lbf_engine* e, void** p, size_t bytes)
+{
+    *p = nullptr;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t r = engine_pool(e->cfg.device, &pool);
+    if (r == cudaSuccess) r = cudaMallocFromPoolAsync(p, bytes, pool, e->stream);
+    if (r == cudaSuccess) e->bytes += bytes;
+    else *p = nullptr;
+    return r;
+}
+
+// Two allocations only make steps faster, the table of pull sources and the
+// resident steps' words.  Where they do not fit the steps run without them, and
+// where something else does not fit beside them they are given back.
+size_t link_bytes(const lbf_engine* e)
+{
+    const size_t tiles = ((size_t)e->nf + kLinkTile - 1) / kLinkTile;
+    return tiles * (kLinkTile * (sizeof(uint4) + sizeof(uint32_t)) + 2 * sizeof(uint4));
+}
+size_t words_bytes(const lbf_engine* e)
+{
+    return 2 * (size_t)(e->Q - 1) * e->nfp * (e->cfg.storage == LBF_STORE_FP64 ? 16 : 8);
+}
+void drop_words(lbf_engine* e)
+{
+    if (!e->words) return;
+    cudaFreeAsync(e->words, e->stream);
+    e->words = nullptr;
+    e->bytes -= words_bytes(e);
+}
+bool drop_optional(lbf_engine* e)
+{
+    if (!e->words && !e->link_table) return false;
+    drop_words(e);
+    if (e->link_table) {
+        cudaFreeAsync(e->link_table, e->stream);
+        e->link_table = nullptr;
+        e->links = Links{};
+        e->bytes -= link_bytes(e);
+    }
+    return true;
+}
+
 template <class T>
 int dalloc(lbf_engine* e, T** p, size_t count)
 {
     *p = nullptr;
     if (count == 0) count = 1;
-    cudaMemPool_t pool = nullptr;
-    cudaError_t r = engine_pool(e->cfg.device, &pool);
-    if (r == cudaSuccess)
-        r = cudaMallocFromPoolAsync(reinterpret_cast<void**>(p), count * sizeof(T), pool, e->stream);
+    void* v = nullptr;
+    cudaError_t r = pool_alloc(e, &v, count * sizeof(T));
+    if (r == cudaErrorMemoryAllocation && drop_optional(e)) {
+        cudaGetLastError();
+        r = pool_alloc(e, &v, count * sizeof(T));
+    }
     if (r != cudaSuccess)
         return fail(e, r == cudaErrorMemoryAllocation ? LBF_ENOMEM : LBF_ECUDA,
                     std::string("cudaMalloc: ") + cudaGetErrorString(r));
-    e->bytes += count * sizeof(T);
+    *p = static_cast<T*>(v);
     return LBF_OK;
+}
+
+// Scratch of one call, outside the pool.
+template <class T>
+cudaError_t temp_alloc(lbf_engine* e, T** p, size_t count)
+{
+    cudaError_t r = cudaMalloc(p, count * sizeof(T));
+    if (r == cudaErrorMemoryAllocation && drop_optional(e)) {
+        cudaGetLastError();
+        cudaMemPool_t pool = nullptr;
+        r = cudaStreamSynchronize(e->stream);
+        if (r == cudaSuccess) r = engine_pool(e->cfg.device, &pool);
+        if (r == cudaSuccess) r = cudaMemPoolTrimTo(pool, 0);
+        if (r == cudaSuccess) r = cudaMalloc(p, count * sizeof(T));
+    }
+    return r;
 }
 
 // Reference lattice tables in reference component order ({y,x} / {z,y,x}),
@@ -256,7 +318,7 @@ void launch_step(lbf_engine* e, bool pull, int out)
         e->sp.seed = dither && pull ? (++e->steps * 2654435761u) | 1u : 0u;
         e->sp.reverse = pull ? (int)(++e->pulls & 1u) : 0;
         ScspLaunch a{grid_of(e), e->force, e->sp, fin, fout, macros_of(e), e->err, e->stream,
-                     e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, Links{e->link_row, e->link_mask, e->link_base}};
+                     e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, e->links};
         launch_scsp(e->D, (int)e->cfg.storage, e->cfg.collision == LBF_MRT, pull, out, a);
     } else {
         // 16-bit storage rounds stochastically with a fresh seed every pull
@@ -472,7 +534,7 @@ int expand_to_host(lbf_engine* e, std::vector<double>& compact)
         return LBF_OK;
     }
     double* tmp = nullptr;
-    LBF_CK(e, cudaMalloc(&tmp, count * sizeof(double)));
+    LBF_CK(e, temp_alloc(e, &tmp, count));
     if (e->D == 3) convert<D3Q19>(e, true, e->f[e->cur], tmp);
     else convert<D2Q9>(e, true, e->f[e->cur], tmp);
     cudaError_t r = cudaGetLastError();
@@ -937,14 +999,6 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
                                                    e->coord, e->node_label, e->node_phase);
     LBF_CUDA(cudaGetLastError());
     LBF_CUDA(cudaMemcpyAsync(e->label_force, lforce.data(), lforce.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream));
-    if (c.model == LBF_MODEL_SCSP && scsp_uses_links(e->D, (int)c.storage)) {
-        const size_t tiles = (count + kLinkTile - 1) / kLinkTile;
-        LBF_ALLOC(e->link_row, tiles * kLinkTile);
-        LBF_ALLOC(e->link_mask, tiles * kLinkTile);
-        LBF_ALLOC(e->link_base, 2 * tiles);
-        launch_build_links(grid_of(e), e->link_row, e->link_mask, e->link_base, e->stream);
-        LBF_CUDA(cudaGetLastError());
-    }
     if (boundaries || c.model == LBF_MODEL_COLOR) {
         if ((rc = ensure_vox(e))) { std::string m = e->last_error; lbf_destroy(e); return fail(nullptr, rc, m); }
     }
@@ -1123,6 +1177,20 @@ int lbf_create(const lbf_config* cfg, const lbf_label labels[256], const uint8_t
         LBF_CUDA(cudaMemcpyAsync(e->tib, tib.data(), tib.size() * sizeof(double), cudaMemcpyHostToDevice, e->stream));
         LBF_CUDA(cudaStreamSynchronize(e->stream));
     }
+    // Last, so that it takes nothing the engine needs.
+    if (c.model == LBF_MODEL_SCSP && scsp_uses_links(e->D, (int)c.storage) && e->nf) {
+        if (pool_alloc(e, &e->link_table, link_bytes(e)) == cudaSuccess) {
+            const size_t tiles = ((size_t)e->nf + kLinkTile - 1) / kLinkTile;
+            uint4* row = static_cast<uint4*>(e->link_table);
+            uint4* base = row + tiles * kLinkTile;
+            uint32_t* mask = reinterpret_cast<uint32_t*>(base + 2 * tiles);
+            launch_build_links(grid_of(e), row, mask, base, e->stream);
+            LBF_CUDA(cudaGetLastError());
+            e->links = Links{row, mask, base};
+        } else {
+            cudaGetLastError();
+        }
+    }
     LBF_CUDA(cudaStreamSynchronize(e->stream));
 #undef LBF_ALLOC
 #undef LBF_CUDA
@@ -1140,7 +1208,7 @@ void lbf_destroy(lbf_engine* e)
                     e->dens, e->angle_id, e->angles, e->tib, e->err, e->partial, e->red_done,
                     e->zh_node, e->zh_code, e->zh_bits, e->zh_value, e->zh_num, e->dense_tmp, e->film_bits[0], e->film_bits[1],
                     e->stage, e->phid, e->solid_f[0], e->solid_f[1], e->words,
-                    e->link_row, e->link_mask, e->link_base};
+                    e->link_table};
     for (void* p : ptrs) if (p) cudaFreeAsync(p, e->stream);
     if (e->stream) cudaStreamSynchronize(e->stream);
     if (e->h_red) cudaFreeHost(e->h_red);
@@ -1263,7 +1331,7 @@ int lbf_block_sums(lbf_engine* e, uint32_t block, double* out, size_t n)
     cudaGetLastError();
     if (on_device && pa.device != e->cfg.device) return fail(e, LBF_EINVAL, "out is device memory of another device");
     double* d = on_device ? out : nullptr;
-    if (!on_device) LBF_CK(e, cudaMalloc(&d, nb * 5 * sizeof(double)));
+    if (!on_device) LBF_CK(e, temp_alloc(e, &d, nb * 5));
     const Grid g = grid_of(e);
     if (e->D == 2) {
         // 2-D: cubes are block x block squares of the single layer.
@@ -1330,31 +1398,28 @@ constexpr uint32_t kResidentSteps = 1024;
 // the launch or the words' memory: the caller then launches step by step.
 bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
 {
-    const size_t bytes = 2 * (size_t)(e->Q - 1) * e->nfp * (e->cfg.storage == LBF_STORE_FP64 ? 16 : 8);
+    // From now on step by step.
+    auto refused = [e] {
+        cudaGetLastError();
+        drop_words(e);
+        e->resident_nodes = 0;
+        return false;
+    };
     bool clear = nsteps >= 0xffffffffu - e->tag;   // step numbers start over: no word may still hold one
     if (!e->words) {
-        unsigned long long* w = nullptr;
-        if (dalloc(e, &w, bytes / 8)) {
-            cudaGetLastError();
-            e->resident_nodes = 0;
-            return false;
-        }
-        e->words = w;
+        if (pool_alloc(e, &e->words, words_bytes(e)) != cudaSuccess) return refused();
         clear = true;
     }
     if (clear) {
-        if (cudaMemsetAsync(e->words, 0, bytes, e->stream) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (cudaMemsetAsync(e->words, 0, words_bytes(e), e->stream) != cudaSuccess) return refused();
         e->tag = 0;
     }
     const bool dither = e->cfg.storage == LBF_STORE_FP16 || e->cfg.storage == LBF_STORE_BF16;
     e->sp.seed = dither ? e->steps + 1 : 0;
     const ScspLaunch a{grid_of(e), e->force, e->sp, e->f[e->cur], e->f[e->cur ^ 1], macros_of(e), e->err, e->stream,
-                       e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, Links{e->link_row, e->link_mask, e->link_base}};
-    if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess) {
-        cudaGetLastError();
-        e->resident_nodes = 0;
-        return false;
-    }
+                       e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, e->links};
+    if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess)
+        return refused();
     e->tag += nsteps;
     if (dither) e->steps += nsteps;
     e->cur ^= 1;
@@ -1457,7 +1522,7 @@ int lbf_set_populations(lbf_engine* e, const double* host, size_t n)
         LBF_CK(e, cudaStreamSynchronize(e->stream));
     } else {
         double* tmp = nullptr;
-        LBF_CK(e, cudaMalloc(&tmp, count * sizeof(double)));
+        LBF_CK(e, temp_alloc(e, &tmp, count));
         cudaError_t r = cudaMemcpyAsync(tmp, compact.data(), count * sizeof(double), cudaMemcpyHostToDevice, e->stream);
         if (r == cudaSuccess) {
             if (e->D == 3) convert<D3Q19>(e, false, e->f[e->cur], tmp);
@@ -1634,7 +1699,7 @@ int lbf_link_mask(lbf_engine* e, uint32_t* host, size_t n)
     int rc = setdev(e);
     if (rc) return rc;
     uint32_t* d = nullptr;
-    LBF_CK(e, cudaMalloc(&d, e->N * sizeof(uint32_t)));
+    LBF_CK(e, temp_alloc(e, &d, e->N));
     const unsigned t = 256;
     const unsigned b = (unsigned)((e->N + t - 1) / t);
     if (e->D == 3) link_mask_kernel<D3Q19><<<b, t, 0, e->stream>>>(grid_of(e), d, e->N);
