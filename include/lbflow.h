@@ -171,6 +171,12 @@ int lbf_darcy_pressure(const double *mob, uint32_t nz, uint32_t ny, uint32_t nx,
  * (LBF_STEP_*) apply to the last step of the call. */
 int lbf_step(lbf_engine *e, uint32_t nsteps, uint32_t flags);
 
+/* Limit, in GPU clock cycles, of a node's wait for its neighbours in a launch of
+ * several steps (unless set about 2 s, four orders above any such wait).  When
+ * it runs out the launch returns and lbf_status shows LBF_ERR_WAIT; the
+ * populations are then undefined until the state is initialised again. */
+int lbf_set_wait_limit(lbf_engine *e, uint64_t cycles);
+
 /* Post-collision populations, dense FP64 [phase][q][voxel], the checkpoint
  * content of saveRst/loadRst (scsp.cpp:277-302; colorfluid.cpp:766-812).
  * Solid voxels are written as 0 and ignored on load.  n = element count. */

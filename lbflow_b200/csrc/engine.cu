@@ -8,6 +8,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -66,6 +67,7 @@ struct lbf_engine {
     uint32_t pulls = 0;             // pull steps launched (alternates the step kernel's node order)
     void* words = nullptr;          // tagged words of the resident steps (optional, allocated on first use)
     uint32_t tag = 0;               // step number of the last resident step
+    long long wait = kResidentWait; // limit of a resident step's waits
     bool resident_asked = false;    // resident_nodes is known
     uint32_t resident_nodes = 0;    // largest geometry the resident steps take
     uint64_t bytes = 0;
@@ -1418,7 +1420,7 @@ bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
     e->sp.seed = dither ? e->steps + 1 : 0;
     const ScspLaunch a{grid_of(e), e->force, e->sp, e->f[e->cur], e->f[e->cur ^ 1], macros_of(e), e->err, e->stream,
                        e->ex[e->cur], e->ex[e->cur ^ 1], out, e->zh, e->links};
-    if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps}) != cudaSuccess)
+    if (launch_scsp_resident(e->D, (int)e->cfg.storage, a, Resident{e->words, e->tag, nsteps, e->wait}) != cudaSuccess)
         return refused();
     e->tag += nsteps;
     if (dither) e->steps += nsteps;
@@ -1426,6 +1428,13 @@ bool resident_steps(lbf_engine* e, uint32_t nsteps, int out)
     return true;
 }
 }  // namespace
+
+int lbf_set_wait_limit(lbf_engine* e, uint64_t cycles)
+{
+    if (!e) return fail(e, LBF_EINVAL, "NULL engine");
+    e->wait = (long long)std::min<uint64_t>(cycles, INT64_MAX);
+    return LBF_OK;
+}
 
 int lbf_step(lbf_engine* e, uint32_t nsteps, uint32_t flags)
 {

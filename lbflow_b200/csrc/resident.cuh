@@ -26,18 +26,21 @@
 //
 // Between launches the populations are in the engine's ordinary array: the
 // first step reads it, the last step writes the other one.  Every wait is
-// bounded; on timeout the kernel sets kErrWait and returns.
+// bounded; on timeout the kernel sets kErrWait and returns, the state is then
+// undefined, and later launches return at their first wait until the state is
+// initialised anew.
 #pragma once
 #include "kernels.cuh"
 
 namespace lbf {
 
-constexpr long long kResidentWait = 4000000000LL;   // clock cycles, about 2 s
+constexpr long long kResidentWait = 4000000000LL;   // default limit of a wait: clock cycles, about 2 s
 
 struct Resident {
     void* words;        // [2][Q - 1][nfp] tagged words
     uint32_t tag0;      // step number before the launch's first step
     uint32_t steps;     // >= 2
+    long long wait;     // limit of a wait, in clock cycles
 };
 
 // A population and the number of the step that wrote it, moved as one access.
@@ -118,13 +121,13 @@ template <class L, class S> struct ResidentBlocks {
     static constexpr int value = L::D == 2 ? (f64 ? 20 : 32) : (f64 ? 16 : 28);
 };
 
-// Whole warp, while waiting: true once the wait has lasted kResidentWait or
-// another block gave up.
-__device__ __forceinline__ bool resident_late(long long& t0, uint32_t* err)
+// Whole warp, while waiting: true once the wait has lasted `limit` or another
+// block gave up.
+__device__ __forceinline__ bool resident_late(long long& t0, long long limit, uint32_t* err)
 {
     const long long t = clock64();
     if (t0 == 0) t0 = t;
-    const bool late = t - t0 > kResidentWait || (*(volatile uint32_t*)err & kErrWait);
+    const bool late = t - t0 >= limit || (*(volatile uint32_t*)err & kErrWait);
     if (!__any_sync(0xffffffffu, late)) return false;
     atomicOr(err, kErrWait);
     return true;
@@ -193,14 +196,14 @@ scsp_resident(const Grid g, const Force F, const ScspParams P0, const typename S
             if constexpr (L::D == 3) {
                 uint32_t n = 0;
                 while (__any_sync(0xffffffffu, miss != 0xffffffffu && PL::peek(dst + miss) != tag))
-                    if ((++n & 255u) == 0 && resident_late(t0, err)) return;
+                    if ((++n & 255u) == 0 && resident_late(t0, r.wait, err)) return;
             }
             miss = 0xffffffffu;
 #pragma unroll
             for (int q = 1; q < L::Q; ++q)
                 if (PL::get(dst + off[q], q, f[q]) != tag) miss = off[q];
             if (!__any_sync(0xffffffffu, miss != 0xffffffffu)) break;
-            if (resident_late(t0, err)) return;
+            if (resident_late(t0, r.wait, err)) return;
         }
     }
     if (live) scsp_store<L, S>(g, P, fout, i, f, nullptr);
