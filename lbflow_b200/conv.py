@@ -138,7 +138,7 @@ def _pack(weight, order, split, flip=False):
     as n and the others as k (flip: the kernel dimensions 2, 3, 4 reversed),
     by one kernel straight from the parameter where it is an fp32 CUDA
     tensor."""
-    if weight.dtype != torch.float32 or not weight.is_cuda:
+    if weight.dtype != torch.float32 or not weight.is_cuda or weight.is_neg():
         w = (weight.flip(2, 3, 4) if flip else weight).permute(order)
         n = math.prod(w.shape[:split])
         mat = w.reshape(n, -1)
@@ -217,15 +217,28 @@ def wgrad(src0, src1, ksize, stride, pad, out_dims, b):
     return out
 
 
+def _rows16(t):
+    """t as contiguous rows that start on a 16-byte boundary."""
+    t = t.contiguous()
+    return t.clone() if t.data_ptr() % 16 else t
+
+
 def _act_grad(gy, y, slope, want_bias):
     """(gradient before the activation as contiguous bf16, bias gradient or
-    None) of the incoming gradient gy; slope None: no activation."""
+    None) of the incoming gradient gy; slope None: no activation.
+
+    By torch operations where the kernel does not apply: other types and
+    channel counts, an output that saved-tensor hooks hand back in another form
+    (its layout may differ, its type or device is left to torch), and a
+    gradient that is itself differentiated."""
     c = gy.shape[-1]
-    if gy.dtype == torch.bfloat16 and gy.is_cuda and gy.numel() and c % 8 == 0 and c <= 2048:
+    fits = (gy.dtype == torch.bfloat16 and gy.is_cuda and gy.numel() and c % 8 == 0 and c <= 2048 and
+            not (gy.requires_grad and torch.is_grad_enabled()) and
+            (slope is None or (y.dtype == torch.bfloat16 and y.device == gy.device and y.shape == gy.shape)))
+    if fits:
         lib = _lib()
-        gy = gy.contiguous()
-        if gy.data_ptr() % 16:
-            gy = gy.clone()
+        gy = _rows16(gy)
+        y = _rows16(y) if slope is not None else None
         out = torch.empty_like(gy) if slope is not None else gy
         if slope is not None or want_bias:
             gb = torch.empty(c, dtype=torch.float32, device=gy.device)
