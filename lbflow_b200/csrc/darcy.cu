@@ -604,12 +604,13 @@ extern "C" int lbf_darcy_pressure(const double* mob, uint32_t nz, uint32_t ny, u
     cudaError_t e = cudaFuncSetAttribute(bottom_cycle, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBottomShared);
     if (e != cudaSuccess) return fail(std::string("lbf_darcy_pressure: ") + cudaGetErrorString(e), LBF_ECUDA);
     cudaMemsetAsync(S.done, 0, sizeof(uint32_t), s);
-    cudaMemsetAsync(phi, 0, n * sizeof(double), s);
     lbf::launch_pdl(setup_fine, nblk(n), kT, s, d0, mob, g, h, S.L[0].mx, S.L[0].my, S.L[0].mz, rhs);
     for (size_t l = 1; l < S.L.size(); ++l)
         lbf::launch_pdl(coarsen_faces, nblk(S.L[l].d.n()), kT, s, S.L[l].d, S.L[l - 1].d, S.L[l - 1].mx, S.L[l - 1].my,
                         S.L[l - 1].mz, S.L[l].mx, S.L[l].my, S.L[l].mz);
-    // Zero-mean right-hand side; phi = 0; r = rhs.
+    // phi = 0, once mob has been read (the caller may pass one array as both);
+    // zero-mean right-hand side; r = rhs.
+    cudaMemsetAsync(phi, 0, n * sizeof(double), s);
     S.sum(n, rhs, nullptr, sc + 4);
     double hr = 0.0;
     lbf::launch_pdl(start_dot, S.nb_dot, kT, s, n, sc + 4, rhs, r, S.L[0].r, S.part, S.done, sc + 3);
