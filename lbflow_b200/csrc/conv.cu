@@ -494,6 +494,10 @@ constexpr size_t conv3_smem(uint32_t groups, uint32_t bn, TapRing r) {
            (2 + 2 * kTapStages) * 8 + 16;
 }
 
+// The epilogue's bf16 rows: a warp's 32, each padded by 16 bytes.
+constexpr uint32_t conv3_pitch(uint32_t bn) { return bn * 2 + 16; }
+constexpr uint32_t conv3_stage_bytes(uint32_t bn) { return kConvProducers * conv3_pitch(bn); }
+
 // G: 8-channel groups held (1, 2, 4 or 8; those past the input's channels are
 // zeros).
 template <int BN, int G>
@@ -652,7 +656,7 @@ conv3_kernel(const __grid_constant__ IgemmArgs p, const uint32_t tx, const uint3
     // tile row, one run in memory.
     const bool vec = p.mode == LBF_OUT_BF16 && p.ld % 8u == 0u && p.n % 8u == 0u;
     const float slope = p.act ? p.slope : 1.f;
-    constexpr uint32_t kPitch = BN * 2u + 16u, kParts = BN / 8u;
+    constexpr uint32_t kPitch = conv3_pitch(BN), kParts = BN / 8u;
     const uint32_t stage = a0 + warp * 32u * kPitch;
 #pragma unroll 1
     for (uint32_t zi = warp >> 2; zi < uint32_t(kCZ); zi += kConvProducers / 128) {
@@ -1041,14 +1045,23 @@ bool conv3_fits(const IgemmArgs& p) {
 
 constexpr int kSmemMost = 227 * 1024;     // shared memory of a block, and of an SM's blocks together
 
+// All 27 taps' weights where that leaves room for three blocks on an SM, else
+// three slots of as many taps as fit into one block's shared memory.  (From 64
+// outputs on tensor memory holds two blocks' accumulators, from 128 on one's: a
+// further block of narrow inputs waits for its turn before it copies anything.)
+constexpr TapRing conv3_ring(uint32_t groups, uint32_t bn) {
+    if (groups == 1 || conv3_smem(groups, bn, TapRing{27, 1}) <= kSmemMost / 3) return TapRing{conv_taps(groups), 1};
+    return conv3_smem(groups, bn, TapRing{3, 3}) <= kSmemMost ? TapRing{3, 3} : TapRing{1, 3};
+}
+
 template <int BN, int G>
 int launch_conv3(const IgemmArgs& p, uint32_t n_pad, cudaStream_t s) {
-    // All 27 taps' weights where that leaves room for three blocks on an SM, else
-    // three slots of as many taps as fit into one block's shared memory.
-    TapRing ring{conv_taps(G), 1};
-    if (G > 1 && conv3_smem(G, BN, ring) > kSmemMost / 3) ring = TapRing{3, 3};
-    if (conv3_smem(G, BN, ring) > kSmemMost) ring = TapRing{1, 3};
-    const size_t sm = conv3_smem(G, BN, ring);
+    constexpr TapRing ring = conv3_ring(G, BN);
+    constexpr size_t sm = conv3_smem(G, BN, ring);
+    static_assert(sm <= size_t(kSmemMost), "a block's shared memory");
+    static_assert(conv_taps(G) % ring.per == 0 && ring.stages <= uint32_t(kTapStages), "whole slots of taps");
+    static_assert(conv3_stage_bytes(BN) <= G * kPlane + ring.per * ring.stages * G * BN * 16u,
+                  "the epilogue's rows go over the tile and the weights, not over the barriers");
     cudaError_t e = cudaFuncSetAttribute(conv3_kernel<BN, G>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMost);
     if (e == cudaSuccess) {
         const uint32_t tx = (p.g.out_w + kCX - 1) / kCX, ty = (p.g.out_h + kCY - 1) / kCY, tz = (p.g.out_d + kCZ - 1) / kCZ;
