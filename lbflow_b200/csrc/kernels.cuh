@@ -293,9 +293,9 @@ __device__ __forceinline__ typename S::R load_pop(const typename S::T* p, int q,
 //                    registers, but most warps take both sides of the split).
 // The indices are the same either way.  Which is faster depends on the
 // kernel: the FP64 single-geometry step (latency-bound at 72 registers) runs
-// 9 % slower uniform; the FP32-arithmetic steps (issue-bound) run 4-12 %
+// 9 % slower uniform; the FP32-arithmetic steps run 4-12 %
 // faster uniform (FP16 storage 28,230 -> 31,230 fluid MLUPS on the 256^3
-// cube) and the batched FP64 step 5 % faster.
+// cube).  The batched steps take the form of the single ones.
 template <class L, bool UNIFORM>
 __device__ __forceinline__ uint32_t pull_sources(const Grid& g, int x, int y, int z, uint32_t (&src)[L::Q])
 {
@@ -358,9 +358,11 @@ __device__ __forceinline__ uint32_t pull_sources(const Grid& g, int x, int y, in
 // The 16-bit storages' steps are bound by instruction issue, and the table
 // saves a seventh of their instructions (FP16: 802 -> 692 per node; 256^3
 // 110.3 -> 100.0 us per step, 192^3 47.9 -> 44.7; BFP16 192^3 55.6 -> 51.5).
-// Wider populations are bound by memory and lose by its 16 bytes per node
-// (FP32 256^3 110.9 -> 112.2, FP64 182 -> 216, where it also spills): they
-// keep the lookups.  For D3Q19 the sources lie in the node's own x-row
+// Wider populations lose by the 16 bytes per node that their gather then waits
+// for (FP32 256^3 110.9 -> 112.2, FP64 182 -> 216, where it also spills) and keep
+// the lookups: FP64 is bound by memory, FP32 by the gather's latency (256^3: 667
+// instructions per node in 64 % of the issue slots, DRAM at 0.73 of the copy
+// bandwidth, long scoreboard the top stall).  For D3Q19 the sources lie in the node's own x-row
 // and eight others, and a row's three sources follow from the compact index of
 // its voxel at x: one less, itself, or itself plus its fluid bit.  The table
 // keeps that index for the eight rows as 16-bit offsets from a per-tile base
@@ -567,9 +569,9 @@ __device__ __forceinline__ float2 dup2(float a) { return make_float2(a, a); }
 
 // The two-rate update in FP32 arithmetic, two opposite pairs per instruction
 // with the packed FP32 operations of sm_100 (__ffma2_rn, __fadd2_rn,
-// __fmul2_rn: each lane rounds as the scalar operation does).  The FP32
-// storages are issue-bound, and this halves the collision's share of the
-// issued instructions.
+// __fmul2_rn: each lane rounds as the scalar operation does).  16-bit storages
+// are issue-bound, FP32 storage not far from it, and this halves the collision's
+// share of the issued instructions.
 template <class L, bool HAS_A>
 __device__ __forceinline__ void collide_trt_x2(float (&f)[L::Q], const float* A, float B, float C, float K,
                                                const float (&u)[3], const float (&F)[3], float uf, float sp,
@@ -758,7 +760,8 @@ __device__ __forceinline__ void scsp_update(const Grid& g, const Force& F, const
 // With boundary nodes in the same launch FP64 takes five (96 registers, no
 // spill): 161x93x117 with two pressure planes, 537 k nodes, 37.4 us per step;
 // four 39.6, six 40.3, seven 47.4 (the boundary update spills), and a call
-// that is not inlined 70.8.
+// that is not inlined 70.8.  Geometries large enough to feel the two missing
+// blocks take the other form (zou_he_inside).
 template <class S> struct StepBlocks { static constexpr int value = 9, boundary = 9; };
 template <> struct StepBlocks<StoreF64> { static constexpr int value = 7, boundary = 5; };
 
