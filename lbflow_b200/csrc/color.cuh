@@ -222,8 +222,16 @@ template <class L> __host__ __device__ inline int normal_code(int n0, int n1, in
 template <class L> constexpr int normal_codes() { return L::D == 3 ? 11 * 11 * 11 : 7 * 7; }
 
 // Pass 1: phase field.  PULL = false reads the node's own values (t = 0).
+// Bound by memory, so by the loads in flight: behind the wait for the previous
+// kernels the compiler left to itself takes 56 registers for FP64 and keeps fewer
+// of a node's 38 loads open than it did without that wait (64 registers; ncu 78 us
+// against 68 on the 128x128x256 medium).  Compiled for eight blocks per SM it takes
+// 64 again: 241.7 -> 235.3 us per step (six blocks 236.7, five 236.9).
+template <class S, bool FILM> struct PhaseBlocks { static constexpr int value = 0; };   // no bound
+template <> struct PhaseBlocks<StoreF64, false> { static constexpr int value = 8; };
+
 template <class L, class S, bool PULL, bool FILM>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, PhaseBlocks<S, FILM>::value)
 color_phase(const Grid g, const Film film, const typename S::T* fin, double2* __restrict__ dens,
             double* __restrict__ phid, uint32_t* __restrict__ err, const double rho_bar)
 {
